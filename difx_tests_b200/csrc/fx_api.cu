@@ -215,6 +215,7 @@ static void free_ctx(fxc_ctx* x)
     cudaFree(x->d_vbits);
     cudaFree(x->d_spec);
     cudaFree(x->d_spec8);
+    cudaFree(x->d_turn);
     cudaFree(x->d_amax);
     cudaFree(x->d_inv);
     cudaFree(x->d_acc);
@@ -350,6 +351,19 @@ int ctx_create(const fxc_config* cfg, fxc_ctx** out, bool group_subbands)
     if ((e = cudaMalloc(&x->d_vbits, sizeof(uint32_t) * (size_t)c.nant * (x->ld / 32))) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&x->d_spec, x->spec_bytes)) != cudaSuccess) return fail(e);
     if ((e = cudaMemset(x->d_spec, 0, x->spec_bytes)) != cudaSuccess) return fail(e);
+    if (x->spec_mode == kSpecF16 && c.fstage != FXC_F_TC16 && c.fstage != FXC_F_TC32) {
+        // the FFT F stage's FP16 output before its corner turn: up to an eighth of the budget (2 GiB), in
+        // equal parts of the chunk; less where that much is not free
+        const size_t slot = G * x->nsig * (size_t)c.nchan * sizeof(uint32_t);
+        size_t part = std::max<size_t>(64, std::min(T, budget / 8 / slot / 64 * 64));
+        for (;; part = std::max<size_t>(64, part / 2 / 64 * 64)) {
+            const size_t n = (T + part - 1) / part;
+            x->turn_T = (int)round_up((T + n - 1) / n, 64);
+            if ((e = cudaMalloc(&x->d_turn, slot * x->turn_T)) == cudaSuccess) break;
+            if (e != cudaErrorMemoryAllocation || part == 64) return fail(e);
+            (void)cudaGetLastError();
+        }
+    }
     if (fp8) {
         const size_t n8 = x->spec_bytes / 2, nsc = (size_t)x->nsb_g * c.nchan * x->nsig;
         if ((e = cudaMalloc(&x->d_spec8, n8)) != cudaSuccess) return fail(e);
@@ -368,9 +382,10 @@ int ctx_create(const fxc_config* cfg, fxc_ctx** out, bool group_subbands)
             return fail(e);
     }
     if ((e = cudaMalloc(&x->d_counts, sizeof(int) * x->npair_ant)) != cudaSuccess) return fail(e);
-    // d_err[0]: tensor-core X wait-expiry code; d_err[1]: input-window misses
-    if ((e = cudaMalloc(&x->d_err, 2 * sizeof(int))) != cudaSuccess) return fail(e);
-    if ((e = cudaMemset(x->d_err, 0, 2 * sizeof(int))) != cudaSuccess) return fail(e);
+    // d_err[0]: tensor-core X wait-expiry code; d_err[1]: input-window misses; d_err[2, 3]: the F stage's
+    // work counter (FArgs::ctr)
+    if ((e = cudaMalloc(&x->d_err, 4 * sizeof(int))) != cudaSuccess) return fail(e);
+    if ((e = cudaMemset(x->d_err, 0, 4 * sizeof(int))) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&x->d_vis, x->vis_bytes)) != cudaSuccess) return fail(e);
 
     // constant tables: per-subband LO, f32 channel angular frequencies (kernel.c:162-166)
@@ -547,19 +562,40 @@ FArgs ctx_fargs(fxc_ctx* x, const uint8_t* d_data, size_t pitch, int ld)
     a.sb_lo = x->d_sblo;
     a.chan_sub = x->d_chan_sub;
     a.chan_step = x->d_chan_step;
+    a.chalf = 2.0 * x->cfg.bw / x->cfg.nchan;
     a.spec = x->d_spec;
     a.rows = x->rows;
     a.T = x->T;
-    a.tb = x->plan_tb;
     a.cpx = x->cfg.iscomplex;
     a.err = x->d_err;
+    a.ctr = x->d_err + 2;
     a.fkind = x->cfg.fstage == FXC_F_AUTO ? FXC_F_FFT32 : x->cfg.fstage;
     return a;
 }
 
-extern "C" {
-
-}  // extern "C"
+cudaError_t ctx_fstage(const fxc_ctx* x, const FArgs& fa, cudaStream_t st, int* nlaunch)
+{
+    if (nlaunch) *nlaunch = 1;
+    if (!x->d_turn) return launch_fstage(x->cfg.nchan, x->spec_mode, fa, st);
+    const int span = fa.tspan ? fa.tspan : fa.T;
+    for (int s0 = 0; s0 < span; s0 += x->turn_T) {
+        FArgs h = fa;
+        h.spec = x->d_turn;
+        h.T = x->turn_T;
+        h.t_base = fa.t_base + s0;
+        h.nfft = std::max(0, std::min(fa.nfft - s0, x->turn_T));
+        h.tspan = std::min(span - s0, x->turn_T);
+        h.amax = nullptr;
+        h.exact8 = x->cfg.xmode == FXC_X_TC_FP8;
+        cudaError_t e = launch_fstage(x->cfg.nchan, kSpecH16, h, st);
+        if (e != cudaSuccess) return e;
+        e = launch_kmajor(x->d_turn, x->turn_T, h.tspan, fa.nsb, x->nsig, x->cfg.nchan, x->rows, fa.spec, fa.T, s0,
+                          fa.amax, st);
+        if (e != cudaSuccess) return e;
+        if (nlaunch) *nlaunch = 2 * (s0 / x->turn_T + 1);
+    }
+    return cudaSuccess;
+}
 
 extern "C" int fxc_debug_xplain_segments(long long ctas, long long slots, int T, int* tseg, int* tlen)
 {
@@ -624,9 +660,11 @@ static int ctx_correlate(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const 
         fa.tspan = std::min(x->T, (fa.nfft + q - 1) / q * q);
         xa.ntk = fa.tspan;
         {
-            StageScope sc(x, 1, 1);
+            StageScope sc(x, 1, 0);
+            int n = 0;
             if (fp8) FXC_CK(cudaMemsetAsync(x->d_amax, 0, sizeof(unsigned) * xa.nsb * xa.nchan * xa.nsig, x->stream));
-            FXC_CK(launch_fstage(x->cfg.nchan, x->spec_mode, fa, x->stream));
+            FXC_CK(ctx_fstage(x, fa, x->stream, &n));
+            x->stage_launches[1] += n;
         }
         {
             StageScope sc(x, 2, fp8 ? 2 : 1);
@@ -949,19 +987,10 @@ int fxc_autotune(fxc_ctx* x, int reps)
         if ((e = cudaEventSynchronize(e1)) != cudaSuccess) return e;
         return cudaEventElapsedTime(ms, e0, e1);
     };
-    cudaError_t err = cudaSuccess;
+    // The F stage has no shape to choose (its slots draw FFT pairs from a counter; the FFT block only sets
+    // a batch's task size): one run leaves the spectra the X stage's variants are timed on.
+    cudaError_t err = ctx_fstage(x, fa, x->stream);
     float best = 1e30f;
-    int best_tb = x->plan_tb;
-    for (int tb : {8, 16, 32}) {
-        fa.tb = tb;
-        float ms = 0.f;
-        err = timeit([&] { return launch_fstage(c.nchan, x->spec_mode, fa, x->stream); }, &ms);
-        if (err != cudaSuccess) break;
-        if (ms < best) {
-            best = ms;
-            best_tb = tb;
-        }
-    }
     int best_alt = x->plan_alt;
     if (err == cudaSuccess && !tc) {
         XArgs xa{};
@@ -972,7 +1001,6 @@ int fxc_autotune(fxc_ctx* x, int reps)
         xa.nchan = c.nchan;
         xa.nsb = x->nsb_g;
         xa.rows = x->rows;
-        best = 1e30f;
         for (int alt : {0, 1}) {
             xa.alt = alt;
             ctx_xsegments(x, xa);
@@ -991,9 +1019,8 @@ int fxc_autotune(fxc_ctx* x, int reps)
         g_last_cuda = (int)err;
         return FXC_ERR_CUDA;
     }
-    x->plan_tb = best_tb;
     x->plan_alt = best_alt;
-    plan_cache_append({fplan_key(c) + " " + std::to_string(best_tb), xplan_key(x->nsig) + " " + std::to_string(best_alt)});
+    plan_cache_append({fplan_key(c) + " " + std::to_string(x->plan_tb), xplan_key(x->nsig) + " " + std::to_string(best_alt)});
     return fxc_reset(x);   // the timing launches accumulated into the visibilities
 }
 

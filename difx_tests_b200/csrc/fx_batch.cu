@@ -4,7 +4,8 @@
 //
 // Each job owns an ordinary context (device input, delay table, spectra chunk,
 // accumulators).  Per round r (spectra chunk r of every job that has one):
-//   one k_fstage_batch launch per F group  {FFT length, npol, spectra precision, FFTs per CTA}
+//   one k_fpair_batch launch per F group {FFT length, npol, spectra layout} of the jobs whose X stage reads
+//   channel-contiguous spectra, one F launch and corner turn per other job
 //   one k_xplain_batch launch per X group  {8-signal blocks, tile variant} (plain form, <= 64 signals),
 //   then one k_xplain_reduce per job of the group cut into time segments (as its single-job path cuts it)
 //   one X launch per remaining job: the FP16 tensor-core X stage, or the plain X stage of
@@ -38,13 +39,13 @@ struct XGroup {
     int nsig8, alt;   // signal blocks of 8 (jobs with the same count share tile plans)
     std::vector<int> jobs;
 };
-enum LaunchKind { kFGroup = 0, kXGroup = 1, kXJob = 2, kXReduce = 3 };
+enum LaunchKind { kFGroup = 0, kXGroup = 1, kXJob = 2, kXReduce = 3, kFJob = 4 };
 struct Launch {       // one launch of the recorded sequence
     int kind;         // LaunchKind
-    int group;        // F / X group, or the job of a kXJob / kXReduce launch
+    int group;        // F / X group, or the job of a kXJob / kXReduce / kFJob launch
     size_t task_off;  // into d_tasks (int4)
     int ntask;
-    int round;        // kXJob / kXReduce: the round (spectra chunk) whose X arguments it takes
+    int round;        // kXJob / kXReduce / kFJob: the round (spectra chunk) whose arguments it takes
 };
 
 thread_local int g_batch_cuda = 0;
@@ -73,8 +74,9 @@ struct fxc_batch {
     cudaStream_t own = nullptr, stream = nullptr;
     std::vector<FGroup> fg;
     std::vector<XGroup> xg;
-    std::vector<int> job_fg, job_xg;   // job_xg -1: the job's X stage is its own launch
-    std::vector<XArgs> xa_host;        // [nrounds][J], for the launches of one job
+    std::vector<int> job_fg, job_xg;   // -1: the job's F / X stage is its own launch
+    std::vector<FArgs> fa_host;        // [nrounds][J], for the launches of one job
+    std::vector<XArgs> xa_host;
     int nrounds = 0;
     // device tables: FArgs [nrounds][J], XArgs [nrounds][J], tasks (int4) for every recorded launch
     FArgs* d_fargs = nullptr;
@@ -124,7 +126,6 @@ static int build_tables(fxc_batch* b)
             a.t_base = r * c->T;
             a.nfft = std::min(c->T, c->cfg.numffts - r * c->T);
             a.tspan = chunk_span(c, r);
-            a.tb = b->fg[b->job_fg[j]].tb;
             fa[(size_t)r * J + j] = a;
         }
         XArgs x{};
@@ -142,6 +143,7 @@ static int build_tables(fxc_batch* b)
             xa[(size_t)r * J + j].ntk = chunk_span(c, r);
         }
     }
+    b->fa_host = fa;
     b->xa_host = xa;
     std::vector<int4> tasks;
     b->launches.clear();
@@ -159,6 +161,8 @@ static int build_tables(fxc_batch* b)
             }
             if (tasks.size() > off) b->launches.push_back({kFGroup, g, off, (int)(tasks.size() - off), r});
         }
+        for (int j = 0; j < J; j++)
+            if (b->job_fg[j] < 0 && r < nchunks(b->ctx[j])) b->launches.push_back({kFJob, j, 0, 0, r});
         for (int g = 0; g < (int)b->xg.size(); g++) {
             const size_t off = tasks.size();
             const int cg = xplain_channel_group(b->xg[g].nsig8 * 8, b->xg[g].alt);
@@ -204,7 +208,9 @@ static int enqueue_launch(fxc_batch* b, const Launch& l)
     if (l.kind == kFGroup) {
         const FGroup& g = b->fg[l.group];
         FB_CK(launch_fstage_batch(g.nchan, g.npol, g.mode, g.tb, b->d_fargs, b->d_tasks + l.task_off, l.ntask,
-                                  b->stream));
+                                  b->ctx[0]->d_err + 2, b->stream));
+    } else if (l.kind == kFJob) {
+        FB_CK(ctx_fstage(b->ctx[l.group], b->fa_host[(size_t)l.round * b->ctx.size() + l.group], b->stream));
     } else if (l.kind == kXGroup) {
         const XGroup& g = b->xg[l.group];
         FB_CK(launch_xplain_batch(g.nsig8 * 8, g.alt, b->d_xargs, b->d_tasks + l.task_off, l.ntask, b->stream));
@@ -218,15 +224,6 @@ static int enqueue_launch(fxc_batch* b, const Launch& l)
                                             : launch_xtc(x, c->d_err, c->nsm, b->stream));
     }
     return FXC_OK;
-}
-
-// FFTs per CTA candidates of an F group: the F16 staging of tb FFTs must fit one CTA's shared memory
-static bool tb_fits(const fxc_batch* b, const FGroup& g, int tb)
-{
-    if (g.mode != kSpecF16) return true;
-    int optin = 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device) != cudaSuccess) return false;
-    return fstage_smem_bytes(g.nchan, g.mode, g.npol, tb) <= (size_t)optin;
 }
 
 // The whole subintegration of every job: delay tables + counts, then the rounds.
@@ -279,14 +276,16 @@ int fxc_batch_create(const fxc_config* cfgs, int njobs, fxc_batch** out)
         int g = -1;
         for (int k = 0; k < (int)b->fg.size(); k++)
             if (b->fg[k].nchan == c->cfg.nchan && b->fg[k].npol == c->cfg.npol && b->fg[k].mode == mode) g = k;
-        if (g < 0) {
-            const auto it = plans.find(fkey(c->cfg.nchan, c->cfg.npol, mode));
-            b->fg.push_back({c->cfg.nchan, c->cfg.npol, mode, it != plans.end() ? it->second : 16, {}});
-            g = (int)b->fg.size() - 1;
-            while (b->fg[g].tb > 4 && !tb_fits(b, b->fg[g], b->fg[g].tb)) b->fg[g].tb /= 2;
+        if (mode != kSpecF16) {
+            if (g < 0) {
+                const auto it = plans.find(fkey(c->cfg.nchan, c->cfg.npol, mode));
+                const int tb = it != plans.end() ? it->second : 16;
+                b->fg.push_back({c->cfg.nchan, c->cfg.npol, mode, tb == 8 || tb == 32 ? tb : 16, {}});
+                g = (int)b->fg.size() - 1;
+            }
+            b->fg[g].jobs.push_back(j);
         }
-        b->fg[g].jobs.push_back(j);
-        b->job_fg.push_back(g);
+        b->job_fg.push_back(g);   // -1 for K-major spectra: its own F launches
         if (c->cfg.xmode != FXC_X_PLAIN_FP32 || c->nsig > 64) {
             b->job_xg.push_back(-1);   // its own X launch
             continue;
@@ -427,13 +426,19 @@ int fxc_batch_launch_count(fxc_batch* b)
         const int st = build_tables(b);
         if (st != FXC_OK) return st;
     }
-    return 2 * (int)b->ctx.size() + (int)b->launches.size();
+    int n = 2 * (int)b->ctx.size() + (int)b->launches.size();
+    for (const Launch& l : b->launches)
+        if (l.kind == kFJob) {   // an F launch and a corner turn per part of the chunk
+            const fxc_ctx* c = b->ctx[l.group];
+            n += 2 * ((chunk_span(c, l.round) + c->turn_T - 1) / c->turn_T) - 1;
+        }
+    return n;
 }
 
 int fxc_batch_get_plan(fxc_batch* b, int job, int* fft_block, int* x_variant)
 {
     if (!b || job < 0 || job >= (int)b->ctx.size()) return FXC_ERR_INVALID;
-    if (fft_block) *fft_block = b->fg[b->job_fg[job]].tb;
+    if (fft_block) *fft_block = b->job_fg[job] >= 0 ? b->fg[b->job_fg[job]].tb : b->ctx[job]->plan_tb;
     if (x_variant) *x_variant = b->job_xg[job] >= 0 ? b->xg[b->job_xg[job]].alt : b->ctx[job]->plan_alt;
     return FXC_OK;
 }
@@ -463,22 +468,6 @@ int fxc_batch_autotune(fxc_batch* b, int reps)
         *ms = 0.f;
         return FXC_OK;
     };
-    for (int g = 0; g < (int)b->fg.size() && st == FXC_OK; g++) {
-        int best = b->fg[g].tb;
-        float best_ms = 1e30f;
-        for (int tb : {8, 16, 32}) {
-            if (!tb_fits(b, b->fg[g], tb)) continue;
-            b->fg[g].tb = tb;
-            b->tables_valid = false;
-            float ms = 0.f;
-            if ((st = time_group(kFGroup, g, &ms)) != FXC_OK) break;
-            if (ms < best_ms) {
-                best_ms = ms;
-                best = tb;
-            }
-        }
-        b->fg[g].tb = best;
-    }
     for (int g = 0; g < (int)b->xg.size() && st == FXC_OK; g++) {
         int best = b->xg[g].alt;
         float best_ms = 1e30f;

@@ -33,11 +33,15 @@ struct fxc_ctx {
     uint32_t* d_vbits = nullptr;
     void* d_spec = nullptr;
     size_t spec_bytes = 0;
-    // F-stage output layout: kSpecF32 [sb][sig][T][chan] (the plain form, and the FP16 tensor-core
+    // X-stage input layout: kSpecF32 [sb][sig][T][chan] (the plain form, and the FP16 tensor-core
     // form of up to 64 signals on the FFT F stage, whose X stage casts to FP16 on the way into the
     // MMA operand: xf32) or kSpecF16 K-major [sb][chan][rows][T] (the other tensor-core forms)
     int spec_mode = 0;
     bool xf32 = false;
+    // kSpecF16 on the FFT F stage: its FP16 output [nsb_g][nsig][turn_T][nchan], turned into d_spec by
+    // k_kmajor turn_T slots at a time (null: the F stage writes d_spec itself)
+    void* d_turn = nullptr;
+    int turn_T = 0;
     uint8_t* d_spec8 = nullptr;   // FP8 form: e4m3 spectra [nsb][nchan][rows][T]
     unsigned* d_amax = nullptr;   // FP8 form: [nsb*nchan][nsig] absmax bits of the chunk
     float* d_inv = nullptr;       // FP8 form: [nsb*nchan][nsig] inverse scales
@@ -80,14 +84,14 @@ struct fxc_ctx {
     std::vector<cudaEvent_t> event_pool;
     double stage_ms[FXC_NSTAGE] = {0, 0, 0, 0};
     long long stage_launches[FXC_NSTAGE] = {0, 0, 0, 0};
-    // launch plan (fxc_set_plan / fxc_autotune / plan cache): FFTs per F-stage CTA, plain X tile variant
+    // launch plan (fxc_set_plan / fxc_autotune / plan cache): FFTs per F-stage task of a batch, plain X tile variant
     int plan_tb = 16;
     int plan_alt = 0;
 };
 
 // Plan cache (file named by FXC_PLAN_CACHE): lines "<key...> <value>", later lines win.
-// Keys: "F <fft> <npol>" FFTs per CTA of the FP32-output F stage, "H <fft> <npol>" of the
-// F16-output F stage, "X <signal blocks of 8>" plain X tile variant.
+// Keys: "F <fft> <npol>" FFTs per F-stage task of the plain form, "H <fft> <npol>" of the tensor-core
+// forms, "X <signal blocks of 8>" plain X tile variant.
 std::map<std::string, int> plan_cache_load();
 void plan_cache_append(const std::vector<std::string>& lines);
 
@@ -102,5 +106,7 @@ int ctx_run_delay_table(fxc_ctx* x, const double* delays, const double* offs, in
                         const double* d_meta = nullptr);
 // F-stage arguments of this context for device input rows d_data of `pitch` bytes
 fx::FArgs ctx_fargs(fxc_ctx* x, const uint8_t* d_data, size_t pitch, int ld);
+// F stage of fa into the layout the context's X stage reads, on stream st; *nlaunch: kernels launched
+cudaError_t ctx_fstage(const fxc_ctx* x, const fx::FArgs& fa, cudaStream_t st, int* nlaunch = nullptr);
 // the plain X stage's time segments for xa (its nsig and alt set): tseg, tlen, part
 void ctx_xsegments(const fxc_ctx* x, fx::XArgs& xa);

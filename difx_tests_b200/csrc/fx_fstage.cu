@@ -1,33 +1,27 @@
-// fx_fstage.cu -- dispatch of the fused F stage by FFT length (kernels in
-// fx_fstage.cuh, one translation unit per length) and the debug unpack export.
+// fx_fstage.cu -- dispatch of the fused F stage by FFT length (kernels in fx_fpair.cuh, one translation
+// unit per length) and the debug unpack export.
 #include "fx_fstage.cuh"
 
 namespace fx {
 
 cudaError_t launch_fstage_256(int mode, const FArgs& a, cudaStream_t st);
 cudaError_t launch_fstage_batch_256(int mode, int npol, int tb, const FArgs* d_jobs, const int4* d_tasks, int ntask,
-                                  cudaStream_t st);
-size_t fstage_smem_256(int mode, int tb, int npol);
+                                  int* ctr, cudaStream_t st);
 cudaError_t launch_fstage_512(int mode, const FArgs& a, cudaStream_t st);
 cudaError_t launch_fstage_batch_512(int mode, int npol, int tb, const FArgs* d_jobs, const int4* d_tasks, int ntask,
-                                  cudaStream_t st);
-size_t fstage_smem_512(int mode, int tb, int npol);
+                                  int* ctr, cudaStream_t st);
 cudaError_t launch_fstage_1024(int mode, const FArgs& a, cudaStream_t st);
 cudaError_t launch_fstage_batch_1024(int mode, int npol, int tb, const FArgs* d_jobs, const int4* d_tasks, int ntask,
-                                  cudaStream_t st);
-size_t fstage_smem_1024(int mode, int tb, int npol);
+                                  int* ctr, cudaStream_t st);
 cudaError_t launch_fstage_2048(int mode, const FArgs& a, cudaStream_t st);
 cudaError_t launch_fstage_batch_2048(int mode, int npol, int tb, const FArgs* d_jobs, const int4* d_tasks, int ntask,
-                                  cudaStream_t st);
-size_t fstage_smem_2048(int mode, int tb, int npol);
+                                  int* ctr, cudaStream_t st);
 cudaError_t launch_fstage_4096(int mode, const FArgs& a, cudaStream_t st);
 cudaError_t launch_fstage_batch_4096(int mode, int npol, int tb, const FArgs* d_jobs, const int4* d_tasks, int ntask,
-                                  cudaStream_t st);
-size_t fstage_smem_4096(int mode, int tb, int npol);
+                                  int* ctr, cudaStream_t st);
 cudaError_t launch_fstage_8192(int mode, const FArgs& a, cudaStream_t st);
 cudaError_t launch_fstage_batch_8192(int mode, int npol, int tb, const FArgs* d_jobs, const int4* d_tasks, int ntask,
-                                  cudaStream_t st);
-size_t fstage_smem_8192(int mode, int tb, int npol);
+                                  int* ctr, cudaStream_t st);
 
 cudaError_t launch_fstage(int nchan, int mode, const FArgs& a, cudaStream_t st)
 {
@@ -41,6 +35,7 @@ cudaError_t launch_fstage(int nchan, int mode, const FArgs& a, cudaStream_t st)
         if (!ftc32_supported(nchan, mode, a)) return cudaErrorInvalidValue;
         return launch_ftc32(mode, a, st);
     }
+    if (mode == kSpecF16) return cudaErrorInvalidValue;   // the FFT kernels store channel-contiguous spectra
     switch (a.cpx ? nchan : 2 * nchan) {   // FFT length: complex samples fill every bin
     case 256: return launch_fstage_256(mode, a, st);
     case 512: return launch_fstage_512(mode, a, st);
@@ -53,34 +48,20 @@ cudaError_t launch_fstage(int nchan, int mode, const FArgs& a, cudaStream_t st)
 }
 
 cudaError_t launch_fstage_batch(int nchan, int npol, int mode, int tb, const FArgs* d_jobs, const int4* d_tasks,
-                                int ntask, cudaStream_t st)
+                                int ntask, int* ctr, cudaStream_t st)
 {
     switch (2 * nchan) {
-    case 256: return launch_fstage_batch_256(mode, npol, tb, d_jobs, d_tasks, ntask, st);
-    case 512: return launch_fstage_batch_512(mode, npol, tb, d_jobs, d_tasks, ntask, st);
-    case 1024: return launch_fstage_batch_1024(mode, npol, tb, d_jobs, d_tasks, ntask, st);
-    case 2048: return launch_fstage_batch_2048(mode, npol, tb, d_jobs, d_tasks, ntask, st);
-    case 4096: return launch_fstage_batch_4096(mode, npol, tb, d_jobs, d_tasks, ntask, st);
-    case 8192: return launch_fstage_batch_8192(mode, npol, tb, d_jobs, d_tasks, ntask, st);
+    case 256: return launch_fstage_batch_256(mode, npol, tb, d_jobs, d_tasks, ntask, ctr, st);
+    case 512: return launch_fstage_batch_512(mode, npol, tb, d_jobs, d_tasks, ntask, ctr, st);
+    case 1024: return launch_fstage_batch_1024(mode, npol, tb, d_jobs, d_tasks, ntask, ctr, st);
+    case 2048: return launch_fstage_batch_2048(mode, npol, tb, d_jobs, d_tasks, ntask, ctr, st);
+    case 4096: return launch_fstage_batch_4096(mode, npol, tb, d_jobs, d_tasks, ntask, ctr, st);
+    case 8192: return launch_fstage_batch_8192(mode, npol, tb, d_jobs, d_tasks, ntask, ctr, st);
     default: return cudaErrorInvalidValue;
     }
 }
 
-size_t fstage_smem_bytes(int nchan, int mode, int npol, int tb)
-{
-    switch (2 * nchan) {
-    case 256: return fstage_smem_256(mode, tb ? tb : 16, npol);
-    case 512: return fstage_smem_512(mode, tb ? tb : 16, npol);
-    case 1024: return fstage_smem_1024(mode, tb ? tb : 16, npol);
-    case 2048: return fstage_smem_2048(mode, tb ? tb : 16, npol);
-    case 4096: return fstage_smem_4096(mode, tb ? tb : 16, npol);
-    case 8192: return fstage_smem_8192(mode, tb ? tb : 16, npol);
-    default: return 0;
-    }
-}
-
-// Debug export of the unpacked (pre-rotation) samples through the same staging
-// and decode code as k_fstage: out[sb][ant][pol][t][n] for n < F, zero where the
+// Debug export of the unpacked (pre-rotation) samples, decoded byte by byte: out[sb][ant][pol][t][n] for n < F, zero where the
 // antenna is invalid for FFT t.
 template <int F>
 __global__ void k_unpack_debug(FArgs args, float* out)

@@ -8,6 +8,7 @@
 //   delay table    DelayEntry [nant][ld]           one entry per (antenna, FFT of the call)
 //   valid bits     u32  [nant][ld/32]              bit t = antenna valid for FFT t
 //   spectra (F32)  f32x2 [nsb][nsig][T][nchan]     plain X stage input, channel-contiguous
+//   spectra (H16)  f16x2 [nsb][nsig][T][nchan]     the FFT F stage's FP16 output, channel-contiguous
 //   spectra (F16)  f16  [nsb][nchan][rows][T]      tensor-core X stage input, K(=time)-major;
 //                                                  row 2*sig = Re, 2*sig+1 = Im, rows padded
 //   spectra (F8)   e4m3 [nsb][nchan][rows][T]      FP8 form: the F16 spectra times 448/absmax
@@ -38,7 +39,7 @@ struct DelayEntry {
     int valid;      // 0/1 (kernel.c:752-756)
 };
 
-enum SpecMode { kSpecF32 = 0, kSpecF16 = 1 };
+enum SpecMode { kSpecF32 = 0, kSpecF16 = 1, kSpecH16 = 2 };
 
 // device error word bits beyond the tensor-core X stage's wait-expiry codes (1..5)
 constexpr int kWindowMiss = 1 << 4;   // an FFT's input was not inside its input window
@@ -56,12 +57,14 @@ struct FArgs {
     const double* sb_lo;        // [nsb] LO per subband, Hz (device)
     const float* chan_sub;      // [stride]     (f32)(2 pi j bw / nchan)       kernel.c:164
     const float* chan_step;     // [nchan/stride] (f32)(2 pi i stride bw / nchan) kernel.c:165
+    double chalf;               // 2 bw / nchan: half-turns per channel and second of fractional delay
     void* spec;                 // spectra buffer (layout per SpecMode)
     int rows;                   // F16 layout: rows per channel (>= 2*nsig)
-    int tb;                     // FFTs per CTA (8, 16 or 32; 0 = 16), chosen by the plan / autotuner
     unsigned* amax;             // F16 layout, FP8 form: running absmax per (sb*nchan + chan, sig), or null
     int tspan;                  // slots [0, tspan) written (>= nfft, multiple of 64; 0 = T)
+    int exact8;                 // FP8 form (H16 spectra): the scalar FFT kernel (fx_fscalar.cuh)
     int cpx;                    // input format: 0 = 2-bit real, 1 = 8-bit complex (FFT length nchan)
+    int* ctr;                   // two zeroed device ints: the F stage's work counter (left zero)
     int* err;                   // device error word (code 6: an input staging wait expired), or null
     int fkind;                  // F-stage arithmetic (FXC_F_FFT32, FXC_F_TC16 or FXC_F_TC32; 0 = FFT32)
 };

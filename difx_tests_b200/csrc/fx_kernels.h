@@ -28,9 +28,11 @@ cudaError_t launch_ftc(const FArgs& a, cudaStream_t st);
 // FP32-grade tensor-core F stage (error-compensated FP16 pairs), same geometry, F16 or F32 layout
 bool ftc32_supported(int nchan, int mode, const FArgs& a);
 cudaError_t launch_ftc32(int mode, const FArgs& a, cudaStream_t st);
-size_t fstage_smem_bytes(int nchan, int mode, int npol, int tb);
+// FP16 spectra [sb][sig][src_T][chan] -> K-major [sb][chan][rows][dst_T] from slot t_off on (fx_kmajor.cu)
+cudaError_t launch_kmajor(const void* src, int src_T, int span, int nsb, int nsig, int nchan, int rows, void* dst,
+                          int dst_T, int t_off, unsigned* amax, cudaStream_t st);
 cudaError_t launch_fstage_batch(int nchan, int npol, int mode, int tb, const FArgs* d_jobs, const int4* d_tasks,
-                                int ntask, cudaStream_t st);
+                                int ntask, int* ctr, cudaStream_t st);
 cudaError_t launch_xplain_reduce(const XArgs& a, cudaStream_t st);
 void xplain_segments(int nsig, int nchan, int nsb, int T, int nsm, int* tseg, int* tlen);
 void xplain_segment_model(long long ctas, long long slots, int T, int* tseg, int* tlen);

@@ -132,7 +132,7 @@ extern "C" int fxc_correlate_noalloc(const fxc_config* cfg, const uint8_t* d_dat
     const int ld = (int)(((size_t)nfft + 127) / 128 * 128);
     const int stride = 1 << ((int)std::log2((double)c.nchan) / 2);
     size_t off = 0;
-    const size_t o_err = off;     off = align256(off + sizeof(int));
+    const size_t o_err = off;     off = align256(off + 4 * sizeof(int));   // error word, -, work counter
     const size_t o_model = off;   off = align256(off + 4 * sizeof(double) * c.nant);
     const size_t o_sblo = off;    off = align256(off + sizeof(double) * c.nsubband);
     const size_t o_csub = off;    off = align256(off + sizeof(float) * stride);
@@ -167,7 +167,7 @@ extern "C" int fxc_correlate_noalloc(const fxc_config* cfg, const uint8_t* d_dat
     NA_CK(cudaMemcpyAsync(scratch + o_sblo, sblo.data(), sblo.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     NA_CK(cudaMemcpyAsync(scratch + o_csub, csub.data(), csub.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     NA_CK(cudaMemcpyAsync(scratch + o_cstep, cstep.data(), cstep.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-    NA_CK(cudaMemsetAsync(scratch + o_err, 0, sizeof(int), st));
+    NA_CK(cudaMemsetAsync(scratch + o_err, 0, 4 * sizeof(int), st));
     NA_CK(cudaMemsetAsync(scratch + o_counts, 0, sizeof(int) * npair_ant, st));
     NA_CK(cudaMemsetAsync(scratch + o_acc, 0, sizeof(float2) * (size_t)c.nsubband * npair * c.nchan, st));
     NA_CK(cudaMemsetAsync(scratch + o_spec, 0, per_slot * T, st));
@@ -193,9 +193,11 @@ extern "C" int fxc_correlate_noalloc(const fxc_config* cfg, const uint8_t* d_dat
     fa.sb_lo = reinterpret_cast<const double*>(scratch + o_sblo);
     fa.chan_sub = reinterpret_cast<const float*>(scratch + o_csub);
     fa.chan_step = reinterpret_cast<const float*>(scratch + o_cstep);
+    fa.chalf = 2.0 * c.bw / c.nchan;
     fa.spec = scratch + o_spec;
     fa.T = (int)T;
     fa.err = reinterpret_cast<int*>(scratch + o_err);
+    fa.ctr = fa.err + 2;
     XArgs xa{};
     xa.spec = scratch + o_spec;
     xa.acc = d_acc;
