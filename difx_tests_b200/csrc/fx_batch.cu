@@ -62,7 +62,7 @@ thread_local int g_batch_cuda = 0;
 // plan-cache keys as the single-job contexts write them ("F" FP32 spectra, "H" FP16)
 std::string fkey(int nchan, int npol, int mode)
 {
-    return std::string(mode == kSpecF16 ? "H " : "F ") + std::to_string(2 * nchan) + " " + std::to_string(npol);
+    return std::string(mode != kSpecF32 ? "H " : "F ") + std::to_string(2 * nchan) + " " + std::to_string(npol);
 }
 std::string xkey(int nsig8) { return "X " + std::to_string(nsig8); }
 
@@ -220,7 +220,7 @@ static int enqueue_launch(fxc_batch* b, const Launch& l)
         fxc_ctx* c = b->ctx[l.group];
         const XArgs& x = b->xa_host[(size_t)l.round * b->ctx.size() + l.group];
         FB_CK(c->cfg.xmode != FXC_X_TC_FP16 ? launch_xplain(x, b->stream)
-              : c->xf32                     ? launch_xtc32(x, c->d_err, c->nsm, b->stream)
+              : c->spec_mode == kSpecH16    ? launch_xtch(x, c->d_err, c->nsm, b->stream)
                                             : launch_xtc(x, c->d_err, c->nsm, b->stream));
     }
     return FXC_OK;

@@ -33,11 +33,10 @@ struct fxc_ctx {
     uint32_t* d_vbits = nullptr;
     void* d_spec = nullptr;
     size_t spec_bytes = 0;
-    // X-stage input layout: kSpecF32 [sb][sig][T][chan] (the plain form, and the FP16 tensor-core
-    // form of up to 64 signals on the FFT F stage, whose X stage casts to FP16 on the way into the
-    // MMA operand: xf32) or kSpecF16 K-major [sb][chan][rows][T] (the other tensor-core forms)
+    // X-stage input layout: kSpecF32 [sb][sig][T][chan] (the plain form), kSpecH16, the same in FP16 (the FP16
+    // tensor-core form of up to 64 signals on the FFT F stage, whose X stage turns the spectra on the
+    // way into the MMA operand) or kSpecF16 K-major [sb][chan][rows][T] (the other tensor-core forms)
     int spec_mode = 0;
-    bool xf32 = false;
     // kSpecF16 on the FFT F stage: its FP16 output [nsb_g][nsig][turn_T][nchan], turned into d_spec by
     // k_kmajor turn_T slots at a time (null: the F stage writes d_spec itself)
     void* d_turn = nullptr;

@@ -877,9 +877,12 @@ template <int F>
 cudaError_t launch_fstage_batch_F(int mode, int npol, int tb, const FArgs* d_jobs, const int4* d_tasks, int ntask,
                                   int* ctr, cudaStream_t st)
 {
-    if (mode != kSpecF32) return cudaErrorInvalidValue;
-    return npol == 2 ? launch_pair_batch<F, kSpecF32, 2>(d_jobs, d_tasks, ntask, tb, ctr, st)
-                     : launch_pair_batch<F, kSpecF32, 1>(d_jobs, d_tasks, ntask, tb, ctr, st);
+    if (mode == kSpecF32)
+        return npol == 2 ? launch_pair_batch<F, kSpecF32, 2>(d_jobs, d_tasks, ntask, tb, ctr, st)
+                         : launch_pair_batch<F, kSpecF32, 1>(d_jobs, d_tasks, ntask, tb, ctr, st);
+    if (mode != kSpecH16) return cudaErrorInvalidValue;
+    return npol == 2 ? launch_pair_batch<F, kSpecH16, 2>(d_jobs, d_tasks, ntask, tb, ctr, st)
+                     : launch_pair_batch<F, kSpecH16, 1>(d_jobs, d_tasks, ntask, tb, ctr, st);
 }
 
 }  // namespace fx

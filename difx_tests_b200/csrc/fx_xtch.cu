@@ -1,30 +1,33 @@
-// fx_xtc32.cu -- tensor-core X stage on FP32 spectra (tcgen05, FP16 inputs cast in shared
-// memory, FP32 accumulation), up to 64 signals.
+// fx_xtch.cu -- tensor-core X stage on channel-contiguous FP16 spectra (tcgen05, FP32 accumulation), up to
+// 64 signals.
 //
 // The same Gram as fx_xtc.cu (per channel G = A A^T over the real-ified, time-major rows
 // A[2s] = Re X_s, A[2s+1] = Im X_s; kernel.c:846 with the conjugation of kernel.c:557-568), but
-// the operand is read from the plain form's FP32 spectra [sb][sig][T][chan], which the FFT F
-// stage writes with channel-contiguous stores.  The FP16 K-major layout the tensor cores need is
-// a corner turn (time-contiguous rows); done in the F stage it costs that stage a shared-memory
-// stage, barriers and a flush per block of FFTs.  Here it is done on the way into the MMA
-// operand: each FP32 value is rounded to FP16 exactly as the F stage would round it
-// (round-to-nearest of Re and Im), and the Gram accumulates the same MMAs in the same order, so
-// the visibilities are bit-identical to fx_xtc.cu on F16 spectra of the same F stage.
+// the operand is read from the FFT F stage's own layout [sb][sig][T][chan] of (Re, Im) half pairs.
+// The K-major layout the tensor cores need is a corner turn (time-contiguous rows); here it is done
+// on the way into the MMA operand, so it costs no pass over HBM.  Values and MMA order are those
+// of fx_xtc.cu on turned spectra, so the visibilities are bit-identical to it.
 //
-// Persistent, warp-specialised CTA per SM; work item = (subband, 4 channels: one 32-byte sector
-// of each spectrum row, so every DRAM sector fetched is used once):
-//   warp 0     TMA producer: box {4 channels, 32 FFTs, nsig signals} of the FP32 spectra
-//              (unswizzled: {Re, Im} of the 4 channels of FFT t of signal s at 1024 s + 32 t)
-//              into a ring of FP32 stages (as many as 128 KB holds: 2 at 64 signals, 4 at 32)
-//   warp 1     MMA issuer: per stage and channel 2 x tcgen05.mma.kind::f16 M128 N128 K16 on the
-//              channel's FP16 tile (A and B descriptors the same tile)
-//   warps 2-9  cast: FP32 stage j -> K half j % 2 (FFTs 32 (j % 2) .. + 31) of the four channels'
-//              FP16 tiles, 128 rows x 64 FFTs, K-major SWIZZLE_128B, rows >= 2 nsig zero; the two
-//              halves of a tile are disjoint, so the cast fills one while the MMAs read the other
-//   warps 10-13 epilogue: tcgen05.ld of the four channels' accumulators (512 TMEM columns), Re/Im
-//              combination, FP32 accumulate into acc[sb][c][pair(i,j)], i <= j; an item is T / 32
-//              stages long, so its epilogue (one accumulator set, not double-buffered) is a small
-//              part of it.
+// Bound by HBM and the stage pipeline's latency: 2 bytes per sample against 65 flop/B.  32 signals x 4
+// subbands x 2048 channels x 31250 FFTs take 7.5 ms (4.4 TB/s); reading FP32 spectra and rounding
+// them here took 12.9 ms for twice the bytes.
+//
+// Persistent, warp-specialised CTA per SM; work item = (subband, CB channels): 8 channels (one whole
+// 32-byte sector of each spectrum row, N = 64 accumulator columns each) up to 32 signals, 4 channels
+// (N = 128) up to 64, which fills the 512 TMEM columns and 64 KB of operand tiles either way; with 4
+// the other half of a sector is the next item's, which another SM reads at the same time (L2):
+//   warp 0     TMA producer: box {CB channels, 32 FFTs, nsig signals} (unswizzled: (Re, Im) of the CB
+//              channels of FFT t of signal s at 4 CB (32 s + t)) into a ring of stages (as many as
+//              128 KB holds, up to 8)
+//   warp 1     MMA issuer: per stage and channel 2 x tcgen05.mma.kind::f16 M128 K16 on the channel's
+//              tile (A and B descriptors the same tile; with 64-row tiles rows 64 .. 127 of A are the
+//              next tile's, whose accumulator lanes nothing reads)
+//   warps 2-9  turn: stage j -> K half j % 2 (FFTs 32 (j % 2) .. + 31) of the CB channels' tiles, 2 nsig
+//              rows x 64 FFTs, K-major SWIZZLE_128B, rows >= 2 nsig zero; the two halves of a tile are
+//              disjoint, so the turn fills one while the MMAs read the other
+//   warps 10-13 epilogue: tcgen05.ld of the CB channels' accumulators, Re/Im combination, FP32
+//              accumulate into acc[sb][c][pair(i,j)], i <= j; an item is T / 32 stages long, so its
+//              epilogue (one accumulator set, not double-buffered) is a small part of it.
 // Every wait is bounded by time; on expiry the CTA records an error code, drains what it
 // issued (again bounded), frees TMEM and returns.
 #include <cuda.h>
@@ -38,24 +41,22 @@
 
 namespace fx {
 
-namespace tcx32 {
+namespace tcxh {
 
-constexpr int BT = 32;                       // FFTs per FP32 stage (a K half of the FP16 tiles)
-constexpr int CB = 4;                        // channels per work item
+constexpr int BT = 32;                       // FFTs per stage (a K half of the tiles)
 constexpr int MAXSIG = 64;
-constexpr int RING_BYTES = 2 * MAXSIG * BT * CB * 8;   // 128 KB of FP32 stages ([sig][t][ch] float2):
-constexpr int MAXS32 = 8;                    // 2 at 64 signals, 4 at 32, up to 8
-constexpr int TILE_BYTES = 128 * 128;        // 128 rows x 64 FP16
-constexpr int NCW = 8;                       // cast warps
-constexpr int NTHREADS = 32 * (2 + NCW + 4);   // producer, MMA, cast, 4 epilogue warps
-constexpr int TMEM_COLS = 512;               // 4 channels x 128 FP32 columns
-constexpr uint32_t kIdesc = tc::idesc_f16(128, 128);
+constexpr int RING_BYTES = 128 * 1024;       // stages of 4 CB BT nsig bytes
+constexpr int MAXST = 8;
+constexpr int TILES_BYTES = 64 * 1024;       // CB tiles of 512 / CB rows x 64 FP16
+constexpr int NTW = 8;                       // turn warps
+constexpr int NTHREADS = 32 * (2 + NTW + 4);   // producer, MMA, turn, 4 epilogue warps
+constexpr int TMEM_COLS = 512;               // CB channels x 512 / CB FP32 columns
 
 struct Smem {
-    alignas(1024) uint8_t f32[RING_BYTES];
-    alignas(1024) uint8_t f16[CB][TILE_BYTES];
-    alignas(8) uint64_t full32[MAXS32];
-    uint64_t empty32[MAXS32];
+    alignas(1024) uint8_t f16[TILES_BYTES];
+    alignas(1024) uint8_t ring[RING_BYTES];  // (also what the last tile's rows 64 .. 127 read)
+    alignas(8) uint64_t full[MAXST];
+    uint64_t empty[MAXST];
     uint64_t full16[2];                      // per K half
     uint64_t empty16[2];
     uint64_t acc_full;
@@ -76,42 +77,40 @@ __device__ __forceinline__ void tma_load_4d(const CUtensorMap* map, uint64_t* ba
         : "memory");
 }
 
-__device__ __forceinline__ uint32_t pack2(float a, float b)
-{
-    const __half2 h = __floats2half2_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
+}  // namespace tcxh
 
-}  // namespace tcx32
-
-// err: 0 ok; 1 a stage-full wait expired (cast or MMA); 2 a stage-free wait expired (producer or
-//      cast); 3 accumulator wait expired; 4 epilogue wait expired; 5 drain expired
-__global__ void __launch_bounds__(tcx32::NTHREADS, 1)
-k_xtc32(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
+// err: 0 ok; 1 a stage-full wait expired (turn or MMA); 2 a stage-free wait expired (producer or
+//      turn); 3 accumulator wait expired; 4 epilogue wait expired; 5 drain expired
+template <int CB>
+__global__ void __launch_bounds__(tcxh::NTHREADS, 1)
+k_xtch(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
 {
     using namespace tc;
-    using namespace tcx32;
+    using namespace tcxh;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &sm.abort;
 
+    constexpr int N = 512 / CB;                   // accumulator columns (and tile rows) of a channel
+    constexpr int TILE_BYTES = N * 128;
+    constexpr uint32_t kIdesc = tc::idesc_f16(128, N);
     const int nsig = a.nsig;
     const int npair = nsig * (nsig + 1) / 2;
-    const int ncq = a.nchan / CB;                 // channel quads per subband
+    const int ncq = a.nchan / CB;                 // channel groups per subband
     const int nitems = a.nsb * ncq;
-    const int nk = (a.ntk ? a.ntk : a.T) / BT;    // FP32 stages per item (even)
-    const uint32_t stage_bytes = (uint32_t)nsig * BT * CB * 8;
-    const int ns32 = min(MAXS32, (int)(RING_BYTES / stage_bytes));   // FP32 stages in flight
+    const int nk = (a.ntk ? a.ntk : a.T) / BT;    // stages per item (even)
+    const uint32_t stage_bytes = (uint32_t)nsig * BT * CB * 4;
+    const int nst = min(MAXST, (int)(RING_BYTES / stage_bytes));   // stages in flight
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < ns32; s++) {
-            mbar_init(&sm.full32[s], 1);
-            mbar_init(&sm.empty32[s], NCW);   // one arrival per cast warp
+        for (int s = 0; s < nst; s++) {
+            mbar_init(&sm.full[s], 1);
+            mbar_init(&sm.empty[s], NTW);   // one arrival per turn warp
         }
         for (int h = 0; h < 2; h++) {
-            mbar_init(&sm.full16[h], NCW);
+            mbar_init(&sm.full16[h], NTW);
             mbar_init(&sm.empty16[h], 1);     // tcgen05.commit of the half's MMAs
         }
         mbar_init(&sm.acc_full, 1);
@@ -121,14 +120,13 @@ k_xtc32(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
         sm.drain_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // rows 2 nsig .. 127 of every FP16 tile stay zero: the cast writes rows below 2 nsig only
+    // rows 2 nsig .. N - 1 of every tile stay zero: the turn writes rows below 2 nsig only
     {
-        const int nz = (128 - 2 * nsig) * 8;   // 16-byte chunks per tile
-        uint8_t* tiles = &sm.f16[0][0];
+        const int nz = (N - 2 * nsig) * 8;   // 16-byte chunks per tile
         for (int i = threadIdx.x; i < CB * nz; i += NTHREADS) {
             const int tile = i / nz;
             const int rem = i - tile * nz;
-            *reinterpret_cast<uint4*>(tiles + (size_t)tile * TILE_BYTES + (2 * nsig + rem / 8) * 128 + (rem % 8) * 16) =
+            *reinterpret_cast<uint4*>(sm.f16 + (size_t)tile * TILE_BYTES + (2 * nsig + rem / 8) * 128 + (rem % 8) * 16) =
                 make_uint4(0u, 0u, 0u, 0u);
         }
         fence_async_smem();
@@ -148,28 +146,28 @@ k_xtc32(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                 const int sb = item / ncq;
                 const int c0 = (item - sb * ncq) * CB;
                 for (int kb = 0; kb < nk; kb++) {
-                    if (!mbar_wait(&sm.empty32[stage], phase ^ 1, abort_flag)) {
+                    if (!mbar_wait(&sm.empty[stage], phase ^ 1, abort_flag)) {
                         if (!*abort_flag) atomicCAS(err, 0, 2);
                         *abort_flag = 1;
                         break;
                     }
-                    mbar_expect_tx(&sm.full32[stage], stage_bytes);
-                    tma_load_4d(&tmap, &sm.full32[stage], sm.f32 + (size_t)stage * stage_bytes, c0, kb * BT, 0, sb);
+                    mbar_expect_tx(&sm.full[stage], stage_bytes);
+                    tma_load_4d(&tmap, &sm.full[stage], sm.ring + (size_t)stage * stage_bytes, c0, kb * BT, 0, sb);
                     issued++;
-                    if (++stage == ns32) {
+                    if (++stage == nst) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
             }
-            // drain: the last ns32 fills are the only ones that may still be in flight
-            for (int s = 0; s < ns32 && issued > 0; s++) {
+            // drain: the last nst fills are the only ones that may still be in flight
+            for (int s = 0; s < nst && issued > 0; s++) {
                 const long long idx = issued - 1 - s;
                 if (idx < 0) break;
-                const int st = (int)(idx % ns32);
-                const uint32_t ph = (uint32_t)((idx / ns32) & 1);
+                const int st = (int)(idx % nst);
+                const uint32_t ph = (uint32_t)((idx / nst) & 1);
                 const unsigned long long t0 = globaltimer();
-                while (!mbar_try(&sm.full32[st], ph)) {
+                while (!mbar_try(&sm.full[st], ph)) {
                     if (globaltimer() - t0 > WAIT_NS) {
                         atomicCAS(err, 0, 5);
                         sm.drain_fail = 1;
@@ -212,8 +210,8 @@ k_xtc32(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                     // K each, +2 in the descriptors' start field)
 #pragma unroll
                     for (int c = 0; c < CB; c++) {
-                        const uint32_t dt = dlo(sm.f16[c]) + 4 * h;
-                        const uint32_t d = tmem + c * 128;
+                        const uint32_t dt = dlo((sm.f16 + c * TILE_BYTES)) + 4 * h;
+                        const uint32_t d = tmem + c * N;
                         umma<false>(d, udesc(dt), udesc(dt), kIdesc, kb > 0 ? 1u : 0u);
                         umma<false>(d, udesc(dt + 2), udesc(dt + 2), kIdesc, 1u);
                     }
@@ -240,28 +238,26 @@ k_xtc32(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
             }
         }
         __syncwarp();
-    } else if (warp < 2 + NCW) {
-        // ------------------------------------------------------------ cast (warps 2 .. 1 + NCW)
-        // Lane t takes FFT t of the stage for signals s = warp - 2, + NCW, ...: two 16-byte reads
-        // of {Re, Im} of the four channels per (s, t).  The 8 lanes of FFTs 8q .. 8q+7 then
-        // transpose through shuffles: lane L writes word L % 4 (FFTs 2w, 2w+1) of the Re (L % 8 < 4)
-        // or Im row of signal s, chunk 4h + q, in each channel's tile (the Re and Im rows' chunks
-        // differ after the swizzle, so the 8 lanes of a group hit 8 banks; groups q and q ^ 1 meet,
-        // so a store takes at most two bank passes).
-        const int t = lane;
-        const int kq = t >> 3;
-        const int w = lane & 3;
-        const int part = (lane >> 2) & 1;                  // 0: Re row, 1: Im row
-        const int srcA = (lane & ~7) + 2 * w;              // lanes of FFTs 8q + 2w, 8q + 2w + 1
-        const uint32_t sel = part ? 0x7632u : 0x5410u;     // high or low halves of (Re, Im) pairs
-        int s32 = 0;
-        uint32_t ph32 = 0;
+    } else if (warp < 2 + NTW) {
+        // ------------------------------------------------------------ turn (warps 2 .. 1 + NTW)
+        // Lane (w, g) takes FFTs 2w, 2w + 1 of 4 channels: two 16-byte reads give the 4 channels' Re and Im
+        // words of K chunk 4h + w / 4 (byte_perm), eight 4-byte stores put them into the tiles.  With 4
+        // channels g picks the signal, s or s + 2; with 8 it is the channel quad, of signal s + 2 (g ^ it)
+        // in step it.  The rows of s and s + 2 differ in bit 2 of the swizzle, so the two half warps
+        // store to different halves of the 32 banks; the reads take the odd FFT first where that
+        // puts a quarter warp on 8 different 16-byte slots.  Each warp takes 4 signals at a time.
+        const int w = CB == 4 ? lane & 15 : lane >> 1;
+        const int g = CB == 4 ? lane >> 4 : lane & 1;
+        const int j = CB == 4 ? (w >> 2) & 1 : (w >> 1) & 1;
+        const uint32_t sre = j ? 0x1054u : 0x5410u, sim = j ? 0x3276u : 0x7632u;
+        int st = 0;
+        uint32_t ph = 0;
         uint32_t ph16 = 0;   // bit h: phase of K half h
         bool stop = false;
         for (int item = blockIdx.x; item < nitems && !stop; item += gridDim.x) {
             for (int kb = 0; kb < nk; kb++) {
                 const int h = kb & 1;
-                if (!mbar_wait_warp(&sm.full32[s32], ph32, abort_flag)) {
+                if (!mbar_wait_warp(&sm.full[st], ph, abort_flag)) {
                     if (lane == 0) {
                         if (!*abort_flag) atomicCAS(err, 0, 1);
                         *abort_flag = 1;
@@ -277,44 +273,46 @@ k_xtc32(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                     stop = true;
                     break;
                 }
-                const uint8_t* src = sm.f32 + (size_t)s32 * stage_bytes;
-                const int k = 4 * h + kq;                      // chunk of the 128-byte tile row
-                // four signals per pass, their reads issued together (the chain read -> shuffles ->
-                // stores of one signal is latency-bound)
-                for (int s0 = warp - 2; s0 < nsig; s0 += 4 * NCW) {
-                    float4 v[4][2];
+                const uint8_t* src = sm.ring + (size_t)st * stage_bytes + (CB == 4 ? 0 : 16 * g);
+                const int k = 4 * h + (w >> 2);                // chunk of the 128-byte tile row
+                constexpr int STEPS = CB == 4 ? 2 : 4;         // (signals, quads) of 4 signals per lane
+                for (int s0 = 4 * (warp - 2); s0 < nsig; s0 += 4 * NTW) {
+                    uint4 v[STEPS][2];
 #pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int s = s0 + NCW * u;
-                        const float4* p = reinterpret_cast<const float4*>(src + s * 1024 + t * 32);
-                        v[u][0] = s < nsig ? p[0] : make_float4(0.f, 0.f, 0.f, 0.f);   // channels c0, c0 + 1
-                        v[u][1] = s < nsig ? p[1] : make_float4(0.f, 0.f, 0.f, 0.f);   // channels c0 + 2, c0 + 3
+                    for (int u = 0; u < STEPS; u++) {
+                        const int s = s0 + (CB == 4 ? u + 2 * g : (u >> 1) + 2 * (g ^ (u & 1)));
+                        const uint4* p = reinterpret_cast<const uint4*>(src + (s * BT + 2 * w) * (4 * CB));
+                        if (s < nsig) {
+                            v[u][0] = p[j * (CB / 4)];
+                            v[u][1] = p[(1 - j) * (CB / 4)];
+                        }
                     }
 #pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int s = s0 + NCW * u;
-                        if (s >= nsig) break;   // warp-uniform: s depends on the warp only
-                        const uint32_t hc[4] = {pack2(v[u][0].x, v[u][0].y), pack2(v[u][0].z, v[u][0].w),
-                                                pack2(v[u][1].x, v[u][1].y), pack2(v[u][1].z, v[u][1].w)};
-                        const int row = 2 * s + part;
-                        const int off = row * 128 + ((k ^ (row & 7)) << 4) + w * 4;
+                    for (int u = 0; u < STEPS; u++) {
+                        const int s = s0 + (CB == 4 ? u + 2 * g : (u >> 1) + 2 * (g ^ (u & 1)));
+                        if (s < nsig) {
+                            const uint32_t x[4] = {v[u][0].x, v[u][0].y, v[u][0].z, v[u][0].w};
+                            const uint32_t y[4] = {v[u][1].x, v[u][1].y, v[u][1].z, v[u][1].w};
+                            const int r0 = 2 * s, r1 = 2 * s + 1;
+                            uint8_t* re = sm.f16 + (CB == 4 ? 0 : 4 * g * TILE_BYTES) + (w & 3) * 4 + r0 * 128 + ((k ^ (r0 & 7)) << 4);
+                            uint8_t* im = sm.f16 + (CB == 4 ? 0 : 4 * g * TILE_BYTES) + (w & 3) * 4 + r1 * 128 + ((k ^ (r1 & 7)) << 4);
 #pragma unroll
-                        for (int c = 0; c < CB; c++) {
-                            const uint32_t x0 = __shfl_sync(0xffffffffu, hc[c], srcA);
-                            const uint32_t x1 = __shfl_sync(0xffffffffu, hc[c], srcA + 1);
-                            *reinterpret_cast<uint32_t*>(sm.f16[c] + off) = __byte_perm(x0, x1, sel);
+                            for (int c = 0; c < 4; c++) {
+                                *reinterpret_cast<uint32_t*>(re + c * TILE_BYTES) = __byte_perm(x[c], y[c], sre);
+                                *reinterpret_cast<uint32_t*>(im + c * TILE_BYTES) = __byte_perm(x[c], y[c], sim);
+                            }
                         }
                     }
                 }
                 fence_async_smem();   // the tiles are read by the tensor cores (async proxy)
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(&sm.empty32[s32]);
+                    mbar_arrive(&sm.empty[st]);
                     mbar_arrive(&sm.full16[h]);
                 }
-                if (++s32 == ns32) {
-                    s32 = 0;
-                    ph32 ^= 1;
+                if (++st == nst) {
+                    st = 0;
+                    ph ^= 1;
                 }
                 ph16 ^= 1u << h;
             }
@@ -339,13 +337,13 @@ k_xtc32(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
             tc_fence_after();
             for (int c = 0; c < CB; c++) {
                 float* out = reinterpret_cast<float*>(acc + ((size_t)sb * a.nchan + c0 + c) * npair);
-                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + c * 128;
+                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + c * N;
 #pragma unroll 1
-                for (int cq = 0; cq < 4; cq++) {      // 32 columns = 16 signal pairs j per chunk
+                for (int cq = 0; cq < N / 32; cq++) {      // 32 columns = 16 signal pairs j per chunk
                     uint32_t v[32];
                     tmem_ld32(taddr + cq * 32, v);
                     tmem_wait_ld();
-                    if (c == CB - 1 && cq == 3) {
+                    if (c == CB - 1 && cq == N / 32 - 1) {
                         tc_fence_before();
                         mbar_arrive(&sm.acc_empty);
                     }
@@ -375,39 +373,44 @@ k_xtc32(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
     }
 }
 
-static size_t xtc32_smem() { return sizeof(tcx32::Smem) + 1024; }
-
-cudaError_t launch_xtc32(const XArgs& a, int* d_err, int nsm, cudaStream_t st)
+template <int CB>
+static cudaError_t launch_xtch_t(const XArgs& a, int* d_err, int nsm, cudaStream_t st)
 {
-    using namespace tcx32;
-    const int nslot = a.ntk ? a.ntk : a.T;
-    if (a.nsig < 1 || a.nsig > MAXSIG || a.nchan < CB || a.nchan % CB != 0 || a.T % BT != 0 || nslot % (2 * BT) != 0 ||
-        nslot > a.T || a.nsb < 1 || !a.spec || !a.acc)
-        return cudaErrorInvalidValue;
-    if (xtc32_smem() > 227 * 1024) return cudaErrorInvalidValue;
+    using namespace tcxh;
     auto enc = tc::tensor_map_encoder();
     if (!enc) return cudaErrorNotSupported;
-    // FP32 spectra [sb][sig][T][chan] (8-byte complex elements): box {4 channels, 32 FFTs, nsig, 1},
-    // unswizzled (dense 16-byte rows: with a swizzle, rows narrower than the swizzle span are each
-    // padded to a whole 128-byte line)
+    // spectra [sb][sig][T][chan] (4-byte complex elements): box {CB channels, 32 FFTs, nsig, 1}, unswizzled
+    // (dense 16- or 32-byte rows: with a swizzle, rows narrower than the swizzle span are each padded
+    // to a whole 128-byte line)
     CUtensorMap map;
     const cuuint64_t dims[4] = {(cuuint64_t)a.nchan, (cuuint64_t)a.T, (cuuint64_t)a.nsig, (cuuint64_t)a.nsb};
-    const cuuint64_t strides[3] = {(cuuint64_t)a.nchan * 8, (cuuint64_t)a.T * a.nchan * 8,
-                                   (cuuint64_t)a.nsig * a.T * a.nchan * 8};
+    const cuuint64_t strides[3] = {(cuuint64_t)a.nchan * 4, (cuuint64_t)a.T * a.nchan * 4,
+                                   (cuuint64_t)a.nsig * a.T * a.nchan * 4};
     const cuuint32_t box[4] = {(cuuint32_t)CB, (cuuint32_t)BT, (cuuint32_t)a.nsig, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_INT64, 4, const_cast<void*>(a.spec), dims, strides, box, estr,
+    CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, const_cast<void*>(a.spec), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-    const size_t sm = xtc32_smem();
+    const size_t sm = sizeof(Smem) + 1024;
     static unsigned configured = 0;
-    cudaError_t e = set_smem_once(k_xtc32, sm, &configured);
+    cudaError_t e = set_smem_once(k_xtch<CB>, sm, &configured);
     if (e != cudaSuccess) return e;
     const long long nitems = (long long)a.nsb * (a.nchan / CB);
     const int grid = nitems < nsm ? (int)nitems : nsm;
-    k_xtc32<<<grid, NTHREADS, sm, st>>>(map, a, d_err);
+    k_xtch<CB><<<grid, NTHREADS, sm, st>>>(map, a, d_err);
     return cudaGetLastError();
+}
+
+cudaError_t launch_xtch(const XArgs& a, int* d_err, int nsm, cudaStream_t st)
+{
+    using namespace tcxh;
+    const int nslot = a.ntk ? a.ntk : a.T;
+    if (a.nsig < 1 || a.nsig > MAXSIG || a.nchan % 8 != 0 || a.nchan < 8 || a.T % BT != 0 || nslot % (2 * BT) != 0 ||
+        nslot > a.T || a.nsb < 1 || !a.spec || !a.acc)
+        return cudaErrorInvalidValue;
+    static_assert(sizeof(Smem) + 1024 <= 227 * 1024, "one CTA's shared memory");
+    return a.nsig <= 32 ? launch_xtch_t<8>(a, d_err, nsm, st) : launch_xtch_t<4>(a, d_err, nsm, st);
 }
 
 }  // namespace fx
