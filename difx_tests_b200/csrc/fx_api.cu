@@ -268,7 +268,8 @@ int ctx_create(const fxc_config* cfg, fxc_ctx** out, bool group_subbands)
     // stages add each chunk's sums to the accumulators once per CTA, so short chunks make them
     // bound by those additions and by each CTA's pipeline fill (the plain X stage at 64 signals
     // x 1024 channels x 8 subbands: 40.9 TFLOP/s at 2 GiB = 504 slots, 48.4 at 16 GiB).
-    // Bytes per FFT slot and subband: f32x2 [sb][sig][T][chan] (plain), f16x2 of the same order (the FP16
+    // Bytes per FFT slot and subband: f32x2 [sb][sig][T][chan] (plain; its tensor-core X stage has the F stage's
+    // two lanes side by side, the same bytes), f16x2 of the first order (the FP16
     // tensor-core form of up to 64 signals on the FFT F stage: its X stage turns while loading),
     // otherwise f16 [sb][chan][rows][T] (the FP8 form adds an e4m3 copy of half that size; its chunk is
     // a multiple of 128 FFTs), written by the tensor-core F stages, or turned from the FFT F stage's
@@ -281,7 +282,9 @@ int ctx_create(const fxc_config* cfg, fxc_ctx** out, bool group_subbands)
         const bool force16 = ts && std::strcmp(ts, "f16") == 0;
         const bool h16 = c.xmode == FXC_X_TC_FP16 && (c.fstage == FXC_F_AUTO || c.fstage == FXC_F_FFT32) &&
                          x->nsig <= 64 && !force16;
-        x->spec_mode = h16 ? kSpecH16 : tc ? kSpecF16 : kSpecF32;
+        x->xsplit = c.xmode == FXC_X_PLAIN_FP32 && (c.fstage == FXC_F_AUTO || c.fstage == FXC_F_FFT32) &&
+                    xsplit_pays(x->nsig, c.nchan, c.nsubband, c.numffts, x->nsm);
+        x->spec_mode = h16 ? kSpecH16 : tc ? kSpecF16 : x->xsplit ? kSpecP32 : kSpecF32;
     }
     const size_t tq = fp8 ? 128 : 64;
     const size_t per_sb = x->spec_mode == kSpecF16 ? (size_t)c.nchan * x->rows * sizeof(uint16_t)
@@ -371,7 +374,7 @@ int ctx_create(const fxc_config* cfg, fxc_ctx** out, bool group_subbands)
         if ((e = cudaMalloc(&x->d_inv, nsc * sizeof(float))) != cudaSuccess) return fail(e);
     }
     if ((e = cudaMalloc(&x->d_acc, x->acc_bytes)) != cudaSuccess) return fail(e);
-    if (c.xmode == FXC_X_PLAIN_FP32) {
+    if (c.xmode == FXC_X_PLAIN_FP32 && !x->xsplit) {
         // segment partials of the plain X stage when its channel groups underfill the SMs
         int tl = 0;
         xplain_segments(x->nsig, c.nchan, c.nsubband, x->T, x->nsm, &x->xseg_max, &tl);
@@ -596,6 +599,11 @@ cudaError_t ctx_fstage(const fxc_ctx* x, const FArgs& fa, cudaStream_t st, int* 
     return cudaSuccess;
 }
 
+extern "C" int fxc_debug_xsplit_pays(int nsig, int nchan, int nsb, int numffts, int nsm)
+{
+    return xsplit_pays(nsig, nchan, nsb, numffts, nsm);
+}
+
 extern "C" int fxc_debug_xplain_segments(long long ctas, long long slots, int T, int* tseg, int* tlen)
 {
     if (!tseg || !tlen || T < 0) return FXC_ERR_INVALID;
@@ -638,6 +646,7 @@ static int ctx_correlate(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const 
     xa.nsb = x->cfg.nsubband;
     xa.rows = x->rows;
     xa.alt = x->plan_alt;
+    xa.ctr = x->d_err + 2;
     ctx_xsegments(x, xa);
     const int nsb = x->cfg.nsubband, G = x->nsb_g;
     const FArgs fall = fa;
@@ -676,7 +685,8 @@ static int ctx_correlate(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const 
                 x8.inv_scale = x->d_inv;
                 FXC_CK(launch_xtc8(x8, x->d_err, x->nsm, x->stream));
             } else {
-                FXC_CK(!tc ? launch_xplain(xa, x->stream)
+                FXC_CK(x->xsplit ? launch_xsplit(xa, x->cfg.npol, x->cfg.iscomplex, x->d_err, x->nsm, x->stream)
+                       : !tc ? launch_xplain(xa, x->stream)
                            : x->spec_mode == kSpecH16 ? launch_xtch(xa, x->d_err, x->nsm, x->stream)
                                      : launch_xtc(xa, x->d_err, x->nsm, x->stream));
             }
@@ -991,7 +1001,7 @@ int fxc_autotune(fxc_ctx* x, int reps)
     cudaError_t err = ctx_fstage(x, fa, x->stream);
     float best = 1e30f;
     int best_alt = x->plan_alt;
-    if (err == cudaSuccess && !tc) {
+    if (err == cudaSuccess && !tc && !x->xsplit) {
         XArgs xa{};
         xa.spec = x->d_spec;
         xa.acc = x->d_acc;

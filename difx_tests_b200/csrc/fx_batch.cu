@@ -8,8 +8,8 @@
 //   channel-contiguous spectra, one F launch and corner turn per other job
 //   one k_xplain_batch launch per X group  {8-signal blocks, tile variant} (plain form, <= 64 signals),
 //   then one k_xplain_reduce per job of the group cut into time segments (as its single-job path cuts it)
-//   one X launch per remaining job: the FP16 tensor-core X stage, or the plain X stage of
-//   more than 64 signals
+//   one X launch per remaining job: the FP16 tensor-core X stage, the plain X stage on the tensor cores
+//   (fx_xsplit.cu) or that of more than 64 signals
 // A grouped launch works through a task table (F: persistent CTAs striding over it; plain X:
 // one CTA per task), so small and large jobs share the
 // machine inside one launch.  The delay tables and baseline counts run first.
@@ -136,6 +136,7 @@ static int build_tables(fxc_batch* b)
         x.nchan = c->cfg.nchan;
         x.nsb = c->cfg.nsubband;
         x.rows = c->rows;
+        x.ctr = c->d_err + 2;
         x.alt = b->job_xg[j] >= 0 ? b->xg[b->job_xg[j]].alt : c->plan_alt;
         if (c->cfg.xmode == FXC_X_PLAIN_FP32) ctx_xsegments(c, x);   // the single-job path's cut
         for (int r = 0; r < nchunks(c); r++) {
@@ -219,9 +220,10 @@ static int enqueue_launch(fxc_batch* b, const Launch& l)
     } else {
         fxc_ctx* c = b->ctx[l.group];
         const XArgs& x = b->xa_host[(size_t)l.round * b->ctx.size() + l.group];
-        FB_CK(c->cfg.xmode != FXC_X_TC_FP16 ? launch_xplain(x, b->stream)
-              : c->spec_mode == kSpecH16    ? launch_xtch(x, c->d_err, c->nsm, b->stream)
-                                            : launch_xtc(x, c->d_err, c->nsm, b->stream));
+        FB_CK(c->xsplit                       ? launch_xsplit(x, c->cfg.npol, 0, c->d_err, c->nsm, b->stream)
+              : c->cfg.xmode != FXC_X_TC_FP16 ? launch_xplain(x, b->stream)
+              : c->spec_mode == kSpecH16      ? launch_xtch(x, c->d_err, c->nsm, b->stream)
+                                              : launch_xtc(x, c->d_err, c->nsm, b->stream));
     }
     return FXC_OK;
 }
@@ -286,7 +288,7 @@ int fxc_batch_create(const fxc_config* cfgs, int njobs, fxc_batch** out)
             b->fg[g].jobs.push_back(j);
         }
         b->job_fg.push_back(g);   // -1 for K-major spectra: its own F launches
-        if (c->cfg.xmode != FXC_X_PLAIN_FP32 || c->nsig > 64) {
+        if (c->cfg.xmode != FXC_X_PLAIN_FP32 || c->nsig > 64 || c->xsplit) {
             b->job_xg.push_back(-1);   // its own X launch
             continue;
         }

@@ -48,6 +48,7 @@ struct fxc_ctx {
     size_t acc_bytes = 0;
     void* d_xpart = nullptr;      // plain form with few channel groups: X-stage segment partial sums
     int xseg_max = 1;             // segments it holds
+    bool xsplit = false;          // plain form: X stage by launch_xsplit
     int* d_counts = nullptr;
     int* d_err = nullptr;   // device-side wait expiry code of the tensor-core X stage
     int nsm = 148;

@@ -740,7 +740,9 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
                     }
                     const float2 ya = cmul(fa, make_float2(y.x.x, y.y.x));
                     const float2 yb = cmul(fb, make_float2(y.x.y, y.y.y));
-                    if constexpr (MODE == kSpecF32) {
+                    if constexpr (MODE == kSpecP32) {   // both lanes side by side (stored or not together)
+                        if (wa) reinterpret_cast<float4*>(oa)[t + NT * e] = make_float4(ya.x, ya.y, yb.x, yb.y);
+                    } else if constexpr (MODE == kSpecF32) {
                         if (wa) reinterpret_cast<float2*>(oa)[t + NT * e] = ya;
                         if (wb) reinterpret_cast<float2*>(ob)[t + NT * e] = yb;
                     } else {
@@ -769,12 +771,14 @@ template <int F, int MODE, int NPOL, bool CPX>
 __device__ __forceinline__ void pair_locate(const FArgs& a, int sb, int ant, int tb0, int p, int span, PairLoc& L)
 {
     using P = PPlan<F, NPOL, CPX>;
-    constexpr size_t EB = MODE == kSpecF32 ? sizeof(float2) : sizeof(__half2);
+    constexpr size_t EB = MODE == kSpecH16 ? sizeof(__half2) : sizeof(float2);
     const int tc = NPOL == 2 ? tb0 + p : tb0 + 2 * p;
     L.row = a.data + ((size_t)sb * a.nant + ant) * a.pitch;
     L.d = a.dtab + (size_t)ant * a.ld + a.t_base + tc;
-    L.out = reinterpret_cast<unsigned char*>(a.spec) +
-            (((size_t)sb * a.nant + ant) * NPOL * a.T + tc) * P::C * EB;
+    // P32: pairs [sb][ant][T][chan][2 polarisations], or [sb][ant][T / 2][chan][2 FFTs] (tc is even)
+    const size_t slot = MODE == kSpecP32 && NPOL == 2 ? ((size_t)sb * a.nant + ant) * NPOL * a.T + 2 * (size_t)tc
+                                                      : ((size_t)sb * a.nant + ant) * NPOL * a.T + tc;
+    L.out = reinterpret_cast<unsigned char*>(a.spec) + slot * P::C * EB;
     L.out_b = (NPOL == 2 ? (size_t)a.T : 1) * P::C * EB;
     L.plo = a.sb_lo + sb;
     L.chalf = a.chalf;
@@ -866,10 +870,14 @@ cudaError_t launch_fstage_F(int mode, const FArgs& a, cudaStream_t st)
     if constexpr (F <= 4096) if (a.cpx) {   // complex FFT length = nchan <= 4096
         if (mode == kSpecF32)
             return a.npol == 2 ? launch_pair<F, kSpecF32, 2, true>(a, st) : launch_pair<F, kSpecF32, 1, true>(a, st);
+        if (mode == kSpecP32)
+            return a.npol == 2 ? launch_pair<F, kSpecP32, 2, true>(a, st) : launch_pair<F, kSpecP32, 1, true>(a, st);
         return a.npol == 2 ? launch_pair<F, kSpecH16, 2, true>(a, st) : launch_pair<F, kSpecH16, 1, true>(a, st);
     }
     if (mode == kSpecF32)
         return a.npol == 2 ? launch_pair<F, kSpecF32, 2, false>(a, st) : launch_pair<F, kSpecF32, 1, false>(a, st);
+    if (mode == kSpecP32)
+        return a.npol == 2 ? launch_pair<F, kSpecP32, 2, false>(a, st) : launch_pair<F, kSpecP32, 1, false>(a, st);
     return a.npol == 2 ? launch_pair<F, kSpecH16, 2, false>(a, st) : launch_pair<F, kSpecH16, 1, false>(a, st);
 }
 
@@ -880,6 +888,9 @@ cudaError_t launch_fstage_batch_F(int mode, int npol, int tb, const FArgs* d_job
     if (mode == kSpecF32)
         return npol == 2 ? launch_pair_batch<F, kSpecF32, 2>(d_jobs, d_tasks, ntask, tb, ctr, st)
                          : launch_pair_batch<F, kSpecF32, 1>(d_jobs, d_tasks, ntask, tb, ctr, st);
+    if (mode == kSpecP32)
+        return npol == 2 ? launch_pair_batch<F, kSpecP32, 2>(d_jobs, d_tasks, ntask, tb, ctr, st)
+                         : launch_pair_batch<F, kSpecP32, 1>(d_jobs, d_tasks, ntask, tb, ctr, st);
     if (mode != kSpecH16) return cudaErrorInvalidValue;
     return npol == 2 ? launch_pair_batch<F, kSpecH16, 2>(d_jobs, d_tasks, ntask, tb, ctr, st)
                      : launch_pair_batch<F, kSpecH16, 1>(d_jobs, d_tasks, ntask, tb, ctr, st);

@@ -8,6 +8,8 @@
 //   delay table    DelayEntry [nant][ld]           one entry per (antenna, FFT of the call)
 //   valid bits     u32  [nant][ld/32]              bit t = antenna valid for FFT t
 //   spectra (F32)  f32x2 [nsb][nsig][T][nchan]     plain X stage input, channel-contiguous
+//   spectra (P32)  f32x2 [nsb][nant][T][nchan][2 pol]  plain form by the tensor cores (fx_xsplit.cu): the F
+//                  or [nsb][nant][T/2][nchan][2 FFTs]  stage's two lanes side by side
 //   spectra (H16)  f16x2 [nsb][nsig][T][nchan]     the FFT F stage's FP16 output, channel-contiguous
 //   spectra (F16)  f16  [nsb][nchan][rows][T]      tensor-core X stage input, K(=time)-major;
 //                                                  row 2*sig = Re, 2*sig+1 = Im, rows padded
@@ -39,7 +41,7 @@ struct DelayEntry {
     int valid;      // 0/1 (kernel.c:752-756)
 };
 
-enum SpecMode { kSpecF32 = 0, kSpecF16 = 1, kSpecH16 = 2 };
+enum SpecMode { kSpecF32 = 0, kSpecF16 = 1, kSpecH16 = 2, kSpecP32 = 3 };
 
 // device error word bits beyond the tensor-core X stage's wait-expiry codes (1..5)
 constexpr int kWindowMiss = 1 << 4;   // an FFT's input was not inside its input window
@@ -83,6 +85,7 @@ struct XArgs {
     // adds the segments to acc in order (tseg <= 1: no segments, CTAs add to acc directly)
     int tseg, tlen;
     void* part;
+    int* ctr;    // two zeroed device ints: the work counter of launch_xsplit (left zero)
 };
 
 }  // namespace fx

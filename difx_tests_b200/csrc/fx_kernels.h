@@ -38,6 +38,11 @@ void xplain_segments(int nsig, int nchan, int nsb, int T, int nsm, int* tseg, in
 void xplain_segment_model(long long ctas, long long slots, int T, int* tseg, int* tlen);
 int xplain_segments_used(const XArgs& a);
 cudaError_t launch_xplain(const XArgs& a, cudaStream_t st);
+// whether the plain form of this geometry takes launch_xsplit (else launch_xplain)
+bool xsplit_pays(int nsig, int nchan, int nsb, int numffts, int nsm);
+// the plain form's sums on the tensor cores, FP32 values as exact FP16 pairs (up to 64 signals); cpx: 8-bit
+// complex input (spectra beyond FP16's range); spectra in the layout kSpecP32
+cudaError_t launch_xsplit(const XArgs& a, int npol, int cpx, int* d_err, int nsm, cudaStream_t st);
 cudaError_t launch_xplain_batch(int nsig, int alt, const XArgs* d_jobs, const int4* d_tasks, int ntask,
                                 cudaStream_t st);
 int xplain_channel_group(int nsig, int alt);

@@ -1,0 +1,575 @@
+// fx_xsplit.cu -- plain X stage on the tensor cores at FP32 grade: every FP32 spectrum value as an FP16 pair,
+// exact products, and sums taken out of the tensor core every 32 FFTs.
+//
+// Per channel V[i][j] = sum_t X_i conj(X_j) (kernel.c:829-854, conjugation of kernel.c:557-568 folded in).  With
+// x = h + l (h = FP16 rounding of x, l of the remainder; 22 bits), rows H = (Re, Im) and H' = (Im, -Re) of the
+// high parts and L = (Re, Im) of the low ones, time as the contraction index,
+//     D = [H; H'] (H + 2 L)^T     upper 64 rows: real part, lower 64: imaginary part,
+//     V = (D + conj(D)^T) / 2 = H H* + H L* + L H*
+// (the l l* term is below FP32 rounding), so the low parts enter one side only.
+//
+// The tensor core adds into its FP32 accumulator by truncation, which adds up: over 1024 FFTs that takes 5e-6
+// off every visibility, over 64 FFTs 5e-7, over 32 (two additions of low parts, two of high ones, twice) 2.5e-7.
+// So D holds 32 FFTs only; then the epilogue warps add it, rounded to nearest, to running sums in their registers,
+// while the MMAs fill the other D, and the mean of what the truncations took, 2^-22, is put back on the way
+// out.  After 2048 FFTs at most the sums go to the accumulators: additions to a small sum round less than to a
+// large one.  Error of the whole correlation against 64 bits, k_xplain / here (without the 2^-22 / D of
+// 16 FFTs with 2^-23 put back, which is 5 % slower):
+//     4 antennas x 2 pol, 128 channels, 100 FFTs                               1.4 / 1.0e-7 (2.7 / 0.9e-7)
+//     23 antennas, 512 channels, 2 subbands, 1037 FFTs                         3.5 / 1.0e-7 (2.8 / 1.3e-7)
+//     16 antennas x 2 pol, 2048 channels, 2 subbands, 8 chunks of 1954 FFTs    1.5 / 1.0e-7 (2.7 / 1.0e-7)
+//     24 antennas x 2 pol, 1024 channels, 3000 FFTs of 8-bit complex samples   1.7 / 1.1e-7 (2.8 / 1.3e-7)
+//     64 antennas, 1024 channels, 4 subbands, 31250 FFTs                       5.8 / 0.9e-7 (2.6 / 1.0e-7)
+//
+// Time of the X stage, k_xplain / here: the second 0.411 / 0.316 ms, the third 25.0 / 14.2, the fourth 1.66 /
+// 0.79, the fifth 88 / 34 ms.
+//
+// What bounds it is the chain of one stage: copy in (HBM: 8 bytes per spectrum value, read once), cast, 16 MMAs
+// (65 cycles each), flush; shared memory carries all of it: the MMAs' operands, the cast's loads and
+// stores, the copies.  12 or 16 cast warps, cast loads straight from global memory, stages of 8 FFTs, sums kept in
+// TMEM and MMAs taken in turns from the four tiles all measured the same or slower.
+//
+// The F stage stores its two lanes side by side for this kernel ([..][chan][2]: two polarisations of an FFT, or
+// two FFTs): rows of 64 bytes for 4 channels.  The copy engine moves boxes of 32-byte rows at 3.7 TB/s,
+// of 64-byte rows at 6.5.
+//
+// Persistent, warp-specialised CTA per SM; work item = (subband, CB channels) over the chunk's FFTs: 4
+// channels for 33 to 64 signals, one per operand tile, or 8 channels up to 32 signals, two per tile (rows
+// H c0, H c1, H' c0, H' c1; the cross blocks of D are not used):
+//   warp 0       TMA producer: box {CB channels, 16 FFTs, all signals} of the FP32 spectra into a ring of stages
+//                (as many as 96 KB holds); it draws the items
+//   warp 1       MMA issuer
+//   warps 4-11   cast: a stage of 16 FFTs -> half h of the 4 tiles' rows (while the MMAs read the other).  A
+//                thread takes a channel and 4 FFTs of one signal (two polarisations: of both) with 16-byte
+//                reads, and stores three 16-byte chunks each, K-major SWIZZLE_128B.  The K order within a chunk
+//                is the thread's own (any order does, the same for both operands); signal s of channel c stands
+//                in row s ^ (8 / CB) c, so the channels of a quarter warp store to different 16-byte slots.
+//   warps 12-19  epilogue: D -> running sums; those through shared memory to acc[sb][pair][chan], one
+//                vector addition per pair and channel (two channels at NS = 32).  Additions to acc straight from
+//                the registers, a value each, took 85 us per item of 64 signals, of an item's 170.
+// Every wait is bounded by time; on expiry the CTA records an error code, drains what it issued (again
+// bounded), frees TMEM and returns.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include <cuda_fp16.h>
+
+#include "fx_common.cuh"
+#include "fx_kernels.h"
+#include "fx_tc.cuh"
+
+namespace fx {
+
+namespace xsp {
+
+constexpr int KS = 2;                        // K16 steps of a stage
+constexpr int BT = 8 * KS;                   // FFTs per stage, a part of the tiles' rows
+constexpr int NQ = 4 / KS;                   // parts: D holds the products of all of them, 32 FFTs
+constexpr int SEG = 2048;                    // FFTs after which the running sums are sent off at the latest
+constexpr int RING_BYTES = 96 * 1024;
+constexpr int VROW = 65;                     // floats per row of an item's sums on their way out (odd: columns on all banks)
+constexpr int MAXST = 16;
+// item numbers handed to the other warps: the producer is at most MAXST stages, the parts of the tiles and
+// two D ahead of the last of them, and an item has two stages or more
+constexpr int NITEM = 16;
+constexpr int NV = 4;                        // tiles
+constexpr int HT = 128 * 128, LT = 64 * 128; // tile bytes: 128 (64) rows x NQ stages of (Re, Im) halves
+constexpr int NCW = 8, NEW = 8;              // cast and epilogue warps
+constexpr int NTHREADS = 32 * (4 + NCW + NEW);   // warp groups: producer and MMA (two warps idle), cast, epilogue
+// registers per thread of the three groups; their sum fits what the block is launched with (96 a thread)
+constexpr int R_ISSUE = 40, R_CAST = 64, R_EPI = 152;
+static_assert(128 * R_ISSUE + 32 * NCW * R_CAST + 32 * NEW * R_EPI <= NTHREADS * 96, "register split");
+constexpr int EC = 16;                       // columns the epilogue reads at a time
+constexpr int TMEM_COLS = 512;               // two D: 4 x 64 columns each
+
+struct Smem {
+    alignas(1024) uint8_t hi[NV * HT];
+    alignas(1024) uint8_t lo[NV * LT];
+    alignas(1024) uint8_t ring[RING_BYTES];
+    alignas(16) float v[128 * VROW];
+    alignas(8) uint64_t full[MAXST];
+    uint64_t empty[MAXST];
+    uint64_t full16[NQ];                     // per part of the tiles
+    uint64_t empty16[NQ];
+    uint64_t d_full[2];                      // per D
+    uint64_t d_empty[2];
+    uint64_t item_full[NITEM];
+    uint64_t drain;
+    int item[NITEM];                         // the CTA's items in order (nitems and more: no further one)
+    uint32_t tmem_base;
+    int abort;
+    int drain_fail;
+};
+
+__device__ __forceinline__ void tma_load_4d(const CUtensorMap* map, uint64_t* bar, void* dst, int x, int y, int z,
+                                            int w)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
+        "[%2];" ::"r"(tc::smem_u32(dst)),
+        "l"(map), "r"(tc::smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+        : "memory");
+}
+
+// bar.red.or over `n` threads on named barrier `id`: true if any thread passed p
+__device__ __forceinline__ bool bar_or(int id, int n, bool p)
+{
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred pi, po;\n\t"
+        "setp.ne.u32 pi, %1, 0;\n\t"
+        "bar.red.or.pred po, %2, %3, pi;\n\t"
+        "selp.u32 %0, 1, 0, po;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)p), "r"(id), "r"(n)
+        : "memory");
+    return r != 0;
+}
+
+__device__ __forceinline__ uint32_t h2(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+
+}  // namespace xsp
+
+// err: 1 a stage-full wait expired (cast or MMA); 2 a stage-free wait expired (producer or cast); 3 accumulator
+//      wait expired; 4 epilogue wait expired; 5 drain expired
+template <int NS, int NPOL, bool CPX>
+__global__ void __launch_bounds__(xsp::NTHREADS, 1)
+k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
+{
+    using namespace tc;
+    using namespace xsp;
+    constexpr int CB = 256 / NS;                      // channels of an item
+    constexpr int CPT = CB / NV;                      // channels per tile
+    constexpr int SWP = 8 / CB;                       // row permutation: signal s of channel c in row s ^ SWP c
+    constexpr uint32_t kIdesc = tc::idesc_f16(128, 64);
+    // FP16 range: 2-bit spectra reach 3.34 x 8192 = 2.7e4; 8-bit complex ones 180 x 4096 = 7.4e5, taken at 2^-5
+    constexpr float scale = CPX ? 0.03125f : 1.f;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    volatile int* abort_flag = &sm.abort;
+
+    const int nsig = a.nsig;
+    const int npair = nsig * (nsig + 1) / 2;
+    const int ncg = a.nchan / CB;                 // channel groups per subband
+    const int nitems = a.nsb * ncg;
+    const int nk = (a.ntk ? a.ntk : a.T) / BT;    // stages per item (a multiple of NQ)
+    const uint32_t stage_bytes = (uint32_t)nsig * BT * CB * 8;
+    const int nst = min(MAXST, (int)(RING_BYTES / stage_bytes));
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < nst; s++) {
+            mbar_init(&sm.full[s], 1);
+            mbar_init(&sm.empty[s], NCW);
+        }
+        for (int h = 0; h < NQ; h++) {
+            mbar_init(&sm.full16[h], NCW);
+            mbar_init(&sm.empty16[h], 1);     // tcgen05.commit of the part's MMAs
+        }
+        for (int c = 0; c < 2; c++) {
+            mbar_init(&sm.d_full[c], 1);
+            mbar_init(&sm.d_empty[c], NEW);
+        }
+        for (int n = 0; n < NITEM; n++) mbar_init(&sm.item_full[n], 1);
+        mbar_init(&sm.drain, 1);
+        sm.abort = 0;
+        sm.drain_fail = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) tmem_alloc(&sm.tmem_base, TMEM_COLS);
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sm.tmem_base;
+
+    // n-th item of the CTA (every lane of the warp; nitems: none, or a wait gave up)
+    auto item_of = [&](int n) -> int {
+        return mbar_wait_warp(&sm.item_full[n % NITEM], (n / NITEM) & 1, abort_flag)
+                   ? *reinterpret_cast<volatile int*>(&sm.item[n % NITEM])
+                   : nitems;
+    };
+    auto fail = [&](int code) {
+        if (!*abort_flag) atomicCAS(err, 0, code);
+        *abort_flag = 1;
+    };
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R_ISSUE));
+        if (warp == 0) {
+            // ------------------------------------------------------------ producer
+            if (lane == 0) {
+                int stage = 0;
+                uint32_t phase = 0;
+                long long issued = 0;
+                // the first item by the block's number, the others from the counter: some SMs get a quarter less
+                // of the memory's rate than others
+                int item = blockIdx.x;
+                for (int n = 0;; n++) {
+                    if (*abort_flag) item = nitems;
+                    sm.item[n % NITEM] = item;
+                    mbar_arrive(&sm.item_full[n % NITEM]);
+                    if (item >= nitems) break;
+                    const int next = nitems > (int)gridDim.x ? (int)gridDim.x + atomicAdd(a.ctr, 1) : nitems;
+                    const int sb = item / ncg;
+                    const int c0 = (item - sb * ncg) * CB;
+                    for (int kb = 0; kb < nk; kb++) {
+                        if (!mbar_wait(&sm.empty[stage], phase ^ 1, abort_flag)) {
+                            fail(2);
+                            break;
+                        }
+                        mbar_expect_tx(&sm.full[stage], stage_bytes);
+                        tma_load_4d(&tmap, &sm.full[stage], sm.ring + (size_t)stage * stage_bytes, 2 * c0,
+                                    kb * (NPOL == 2 ? BT : BT / 2), 0, sb);
+                        issued++;
+                        if (++stage == nst) {
+                            stage = 0;
+                            phase ^= 1;
+                        }
+                    }
+                    item = next;
+                }
+                if (nitems > (int)gridDim.x) {   // the last CTA to have drawn leaves the counter zero
+                    __threadfence();
+                    if (atomicAdd(a.ctr + 1, 1) == (int)gridDim.x - 1) {
+                        a.ctr[0] = 0;
+                        a.ctr[1] = 0;
+                    }
+                }
+                // drain: the last nst fills are the only ones that may still be in flight
+                for (int s = 0; s < nst && issued > 0; s++) {
+                    const long long idx = issued - 1 - s;
+                    if (idx < 0) break;
+                    if (!mbar_drain(&sm.full[(int)(idx % nst)], (uint32_t)((idx / nst) & 1))) {
+                        atomicCAS(err, 0, 5);
+                        sm.drain_fail = 1;
+                        break;
+                    }
+                }
+            }
+        } else if (warp == 1) {
+            // ------------------------------------------------------------ MMA issuer
+            const uint32_t dsm = (uint32_t)umma_desc(smem_u32(&sm));
+            uint32_t ph = 0;      // phase of the parts of the tiles (one turn for all of them)
+            int db = 0;           // the D of these 32 FFTs, and its phase
+            uint32_t dph = 0;
+            bool ok = true;
+            for (int n = 0; ok; n++) {
+                if (item_of(n) >= nitems) break;
+                for (int kb = 0; kb < nk && ok; kb += NQ) {
+                    if (!mbar_wait_warp(&sm.d_empty[db], dph ^ 1, abort_flag)) {
+                        if (lane == 0) fail(3);
+                        ok = false;
+                    }
+#pragma unroll
+                    for (int h = 0; h < NQ; h++) {
+                        if (ok && !mbar_wait_warp(&sm.full16[h], ph, abort_flag)) {
+                            if (lane == 0) fail(1);
+                            ok = false;
+                        }
+                        tc_fence_after();
+                        if (ok && elect_one()) {
+                            const uint32_t d0 = tmem + db * 256;
+                            uint32_t ds = dsm;
+                            asm volatile("" : "+r"(ds));   // the descriptors are added up here, not kept
+#pragma unroll
+                            for (int c = 0; c < NV; c++)
+#pragma unroll
+                                for (int k = 0; k < 2 * KS; k++) {   // the low parts' steps, then the high ones'
+                                    // a K16 step: 32 bytes of the rows, + 2 in the descriptors' start field
+                                    const int at = 2 * (KS * h + k % KS);
+                                    const uint32_t dh = ds + (uint32_t)((offsetof(Smem, hi) + c * HT) >> 4) + at;
+                                    const uint32_t dl = ds + (uint32_t)((offsetof(Smem, lo) + c * LT) >> 4) + at;
+                                    if (h == 0 && k == 0) umma_ss_acc<false>(d0 + c * 64, udesc(dh), udesc(dl), kIdesc);
+                                    else umma_ss_acc<true>(d0 + c * 64, udesc(dh), udesc(k < KS ? dl : dh), kIdesc);
+                                }
+                            umma_commit(&sm.empty16[h]);
+                            if (h == NQ - 1) umma_commit(&sm.d_full[db]);
+                        }
+                        __syncwarp();
+                    }
+                    dph ^= db;
+                    db ^= 1;
+                    ph ^= 1;
+                }
+            }
+            // drain: every issued MMA retires before TMEM is freed (committed by the issuing lane)
+            if (elect_one()) {
+                umma_commit(&sm.drain);
+                if (!mbar_drain(&sm.drain, 0)) {
+                    atomicCAS(err, 0, 5);
+                    sm.drain_fail = 1;
+                }
+            }
+            __syncwarp();
+        }
+    } else if (warp < 4 + NCW) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R_CAST));
+        // ------------------------------------------------------------ cast
+        const int c = lane & (CB - 1);
+        constexpr int NG = 2 * KS;                        // 16-byte chunks of a row and stage, one per thread
+        const int tg = (lane / CB) & (NG - 1);
+        constexpr int UPW = 32 / (NG * CB);               // units (a signal, or an antenna's two) of a warp at a time
+        const int u0 = (warp - 4) * UPW + lane / (NG * CB);
+        const int nunit = nsig / NPOL;
+        // two channels of a tile at NS = 32: rows H c0, H c1, H' c0, H' c1, so that its first 64 rows are B
+        uint8_t* hi = sm.hi + (c / CPT) * HT + (c % CPT) * 32 * 128;
+        uint8_t* lo = sm.lo + (c / CPT) * LT + (c % CPT) * 32 * 128;
+        // one signal's four values into row s ^ SWP c, chunk NG h + tg
+        auto put = [&](const float2 (&x)[4], int s, int h) {
+            uint32_t hw[4], gw[4], lw[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 v = CPX ? make_float2(x[i].x * scale, x[i].y * scale) : x[i];
+                const __half2 hh = __floats2half2_rn(v.x, v.y);
+                const float2 f = __half22float2(hh);
+                const float2 l = __fadd2_rn(v, make_float2(-f.x, -f.y));
+                const __half2 ll = __floats2half2_rn(l.x, l.y);
+                hw[i] = h2(hh);
+                gw[i] = __byte_perm(hw[i], 0u, 0x1032) ^ 0x80000000u;   // (Im, -Re)
+                lw[i] = h2(__hadd2(ll, ll));
+            }
+            const int r = s ^ (SWP * c);
+            const int off = r * 128 + (((NG * h + tg) ^ (r & 7)) << 4);
+            *reinterpret_cast<uint4*>(hi + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+            *reinterpret_cast<uint4*>(hi + 64 * 128 + off) = make_uint4(gw[0], gw[1], gw[2], gw[3]);
+            *reinterpret_cast<uint4*>(lo + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+        };
+        int st = 0;
+        uint32_t ph = 0;
+        uint32_t ph16 = 0;   // phase of the parts
+        bool stop = false;
+        for (int n = 0; !stop; n++) {
+            if (item_of(n) >= nitems) break;
+            for (int kb = 0; kb < nk; kb++) {
+                const int h = kb & (NQ - 1);
+                if (!mbar_wait_warp(&sm.full[st], ph, abort_flag)) {
+                    if (lane == 0) fail(1);
+                    stop = true;
+                    break;
+                }
+                if (!mbar_wait_warp(&sm.empty16[h], ph16 ^ 1, abort_flag)) {
+                    if (lane == 0) fail(2);
+                    stop = true;
+                    break;
+                }
+                const float4* src = reinterpret_cast<const float4*>(sm.ring + (size_t)st * stage_bytes) + tg * CB + c;
+#pragma unroll 2
+                for (int u = u0; u < nunit; u += NCW * UPW) {
+                    if constexpr (NPOL == 2) {   // [ant][BT][chan] of both polarisations: FFTs tg + NG i
+                        float4 y[4];
+#pragma unroll
+                        for (int i = 0; i < 4; i++) y[i] = src[(u * BT + NG * i) * CB];
+                        const float2 p0[4] = {{y[0].x, y[0].y}, {y[1].x, y[1].y}, {y[2].x, y[2].y}, {y[3].x, y[3].y}};
+                        const float2 p1[4] = {{y[0].z, y[0].w}, {y[1].z, y[1].w}, {y[2].z, y[2].w}, {y[3].z, y[3].w}};
+                        put(p0, 2 * u, h);
+                        put(p1, 2 * u + 1, h);
+                    } else {                     // [sig][BT / 2][chan] of both FFTs of a pair: pairs tg, tg + NG
+                        const float4 y0 = src[u * (BT / 2) * CB], y1 = src[(u * (BT / 2) + NG) * CB];
+                        const float2 x[4] = {{y0.x, y0.y}, {y0.z, y0.w}, {y1.x, y1.y}, {y1.z, y1.w}};
+                        put(x, u, h);
+                    }
+                }
+                fence_async_smem();   // the tiles are read by the tensor cores (async proxy)
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&sm.empty[st]);
+                    mbar_arrive(&sm.full16[h]);
+                }
+                if (++st == nst) {
+                    st = 0;
+                    ph ^= 1;
+                }
+                if (h == NQ - 1) ph16 ^= 1;
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R_EPI));
+        // ------------------------------------------------------------ epilogue
+        const int q = warp & 3;                  // TMEM lane quadrant of this warp
+        const int e = (warp - 4 - NCW) >> 2;     // tiles e and e + 2
+        // columns of this warp's rows: all 64 signals, or the 32 of its own channel of the tile
+        constexpr int NCOL = NS;
+        const uint32_t lane0 = ((uint32_t)(q * 32) << 16) + (NS == 32 ? 32 * (q & 1) : 0);
+        constexpr float inv = 0.5f / (scale * scale) * (1.f + 0x1p-22f);   // what truncation took put back
+        const int nseg = (nk * BT + SEG - 1) / SEG;
+        const int nd = nk / NQ;
+        const int dseg = (nd + nseg - 1) / nseg;      // D per segment of an item
+        int db = 0;
+        uint32_t dph = 0;
+        bool stop = false;
+        for (int nit = 0; !stop; nit++) {
+            const int item = item_of(nit);
+            // all of these warps leave together (a wait may have given up in one of them)
+            if (bar_or(1, 32 * NEW, item >= nitems)) break;
+            const int sb = item / ncg;
+            const int c0 = (item - sb * ncg) * CB;
+            for (int d = 0; d < nd && !stop;) {
+                float2 sum[2][NCOL / 2];
+#pragma unroll
+                for (int t = 0; t < 2; t++)
+#pragma unroll
+                    for (int k = 0; k < NCOL / 2; k++) sum[t][k] = make_float2(0.f, 0.f);
+                for (const int dend = min(d + dseg, nd); d < dend; d++) {
+                    if (!mbar_wait_warp(&sm.d_full[db], dph, abort_flag)) {
+                        if (lane == 0) fail(4);
+                        stop = true;
+                        break;
+                    }
+                    tc_fence_after();
+#pragma unroll
+                    for (int t = 0; t < 2; t++)
+#pragma unroll
+                        for (int n = 0; n < NCOL; n += EC) {
+                            uint32_t v[EC];
+                            tmem_ld16(tmem + lane0 + db * 256 + (e + 2 * t) * 64 + n, v);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int k = 0; k < EC; k += 2)
+                                sum[t][(n + k) / 2] = __fadd2_rn(
+                                    sum[t][(n + k) / 2], make_float2(__uint_as_float(v[k]), __uint_as_float(v[k + 1])));
+                        }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sm.d_empty[db]);
+                    dph ^= db;
+                    db ^= 1;
+                }
+                // ---- sums to the accumulators, a tile at a time (two tiles at NS = 32, one beside the other)
+                // through shared memory: V[i][j] needs D[i][j] and D[j][i], real and imaginary rows
+#pragma unroll
+                for (int t = 0; t < 2; t++) {
+#pragma unroll
+                    for (int ee = 0; ee < (NS == 32 ? 1 : 2); ee++) {
+                        if (NS == 32 || e == ee) {
+                            float* out = sm.v + (q * 32 + lane) * VROW + (NS == 32 ? 32 * e : 0);
+#pragma unroll
+                            for (int n = 0; n < NCOL; n += 2) {
+                                out[n] = sum[t][n / 2].x;
+                                out[n + 1] = sum[t][n / 2].y;
+                            }
+                        }
+                        stop = bar_or(1, 32 * NEW, stop);
+                        if (!stop) {
+                            const int w = 4 * e + q;   // 0 .. 7
+                            float2* acc = reinterpret_cast<float2*>(a.acc) + (size_t)sb * npair * a.nchan + c0;
+                            if constexpr (NS == 32) {
+                                // channels 4 t + g, g = 0 .. 3: tile 2 t + (g >> 1)'s half g & 1; a thread takes channels
+                                // 4 t + 2 x and the next
+                                const int x = w & 1;
+                                for (int i = w >> 1; i < nsig; i += 4) {
+                                    const int j = lane;
+                                    if (j >= i && j < nsig) {
+                                        float r[4];
+#pragma unroll
+                                        for (int y = 0; y < 2; y++) {
+                                            const int k = SWP * (4 * t + 2 * x + y);
+                                            const float* re = sm.v + 32 * y * VROW + 32 * x;
+                                            const float* ig = re + 64 * VROW;
+                                            r[2 * y] = inv * (re[(i ^ k) * VROW + (j ^ k)] + re[(j ^ k) * VROW + (i ^ k)]);
+                                            r[2 * y + 1] = inv * (ig[(i ^ k) * VROW + (j ^ k)] - ig[(j ^ k) * VROW + (i ^ k)]);
+                                        }
+                                        const int p = i * nsig - i * (i - 1) / 2 + (j - i);
+                                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(
+                                                         acc + (size_t)p * a.nchan + 4 * t + 2 * x),
+                                                     "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3])
+                                                     : "memory");
+                                    }
+                                }
+                            } else {
+                                const int ch = ee + 2 * t, k = SWP * ch;
+                                for (int i = w; i < nsig; i += 8)
+                                    for (int j = (i & ~31) + lane; j < nsig; j += 32)
+                                        if (j >= i) {
+                                            const float* re = sm.v;
+                                            const float* ig = sm.v + 64 * VROW;
+                                            const float vr = inv * (re[(i ^ k) * VROW + (j ^ k)] + re[(j ^ k) * VROW + (i ^ k)]);
+                                            const float vm = inv * (ig[(i ^ k) * VROW + (j ^ k)] - ig[(j ^ k) * VROW + (i ^ k)]);
+                                            const int p = i * nsig - i * (i - 1) / 2 + (j - i);
+                                            asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(
+                                                             acc + (size_t)p * a.nchan + ch),
+                                                         "f"(vr), "f"(vm)
+                                                         : "memory");
+                                        }
+                            }
+                        }
+                        stop = bar_or(1, 32 * NEW, stop);
+                    }
+                }
+            }
+        }
+    }
+
+    __syncthreads();
+    // after an expired drain, MMAs may still write TMEM: it stays allocated (code 5 was recorded;
+    // the context's later tensor-core launches cannot be trusted and the process should reset)
+    if (warp == 0 && !sm.drain_fail) {
+        tc_fence_after();
+        tmem_dealloc(tmem, TMEM_COLS);
+    }
+}
+
+template <int NS, int NPOL, bool CPX>
+static cudaError_t launch_xsplit_t(const XArgs& a, int* d_err, int nsm, cudaStream_t st)
+{
+    using namespace xsp;
+    constexpr int CB = 256 / NS;
+    auto enc = tc::tensor_map_encoder();
+    if (!enc) return cudaErrorNotSupported;
+    // spectra [sb][ant][T][chan][2 polarisations] or [sb][sig][T / 2][chan][2 FFTs] of 8-byte complex values
+    CUtensorMap map;
+    const cuuint64_t nt = NPOL == 2 ? a.T : a.T / 2, nr = a.nsig / NPOL, row = (cuuint64_t)a.nchan * 16;
+    const cuuint64_t dims[4] = {(cuuint64_t)2 * a.nchan, nt, nr, (cuuint64_t)a.nsb};
+    const cuuint64_t strides[3] = {row, nt * row, nr * nt * row};
+    const cuuint32_t box[4] = {2 * CB, NPOL == 2 ? BT : BT / 2, (cuuint32_t)nr, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_INT64, 4, const_cast<void*>(a.spec), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+    const size_t sm = sizeof(Smem) + 1024;
+    static unsigned configured = 0;
+    cudaError_t e = set_smem_once(k_xsplit<NS, NPOL, CPX>, sm, &configured);
+    if (e != cudaSuccess) return e;
+    const long long nitems = (long long)a.nsb * (a.nchan / CB);
+    const int grid = nitems < nsm ? (int)nitems : nsm;
+    k_xsplit<NS, NPOL, CPX><<<grid, NTHREADS, sm, st>>>(map, a, d_err);
+    return cudaGetLastError();
+}
+
+template <int NS, int NPOL>
+static cudaError_t launch_xsplit_n(const XArgs& a, int cpx, int* d_err, int nsm, cudaStream_t st)
+{
+    return cpx ? launch_xsplit_t<NS, NPOL, true>(a, d_err, nsm, st) : launch_xsplit_t<NS, NPOL, false>(a, d_err, nsm, st);
+}
+
+// A geometry-only rule (a batch's jobs take the same path as alone).  The kernel's time is that of an item,
+// 10 us + 0.042 (2 signals) to 0.07 us (64) per FFT, times the items over the SMs; k_xplain's grows with the
+// multiply-adds but takes 23 us or more.  Measured k_xplain / here, us (items):
+//   9 to 64 signals, items for most SMs: here the faster one for every number of FFTs tried
+//       4096 FFTs, 9 signals (128 items) 210 / 204; 32 (128) 441 / 267; 33 (128) 400 / 235; 64 (512) 5683 / 2143
+//       and below, not: 9 (64) 117 / 203; 32 (96) 325 / 267; 33 (64) 206 / 234; 1024 FFTs, 9 (64) 41 / 59
+//   up to 8 signals k_xplain has little to do: 4096 FFTs (512) 290 / 699
+//   short calls of one item per SM: 64 FFTs, 2 signals (16) 23 / 13; 8 (128) 33 / 14; 64 (64) 45 / 23;
+//       not with more items: 2 (512) 24 / 25
+bool xsplit_pays(int nsig, int nchan, int nsb, int numffts, int nsm)
+{
+    if (nsig < 1 || nsig > 64 || nchan < 8 || nchan % 8 != 0) return false;
+    const long long nitems = (long long)nsb * (nchan / (nsig <= 32 ? 8 : 4));
+    if (numffts <= 128 && nitems <= nsm) return true;
+    return nsig > 8 && nitems * 7 >= (long long)nsm * 6;
+}
+
+cudaError_t launch_xsplit(const XArgs& a, int npol, int cpx, int* d_err, int nsm, cudaStream_t st)
+{
+    using namespace xsp;
+    const int nslot = a.ntk ? a.ntk : a.T;
+    if (a.nsig < 1 || a.nsig > 64 || a.nsig % npol || a.nchan % 8 != 0 || a.nchan < 8 || a.T % BT != 0 || nslot < 1 ||
+        nslot % (NQ * BT) != 0 || nslot > a.T || a.nsb < 1 || !a.spec || !a.acc)
+        return cudaErrorInvalidValue;
+    static_assert(sizeof(Smem) + 1024 <= 227 * 1024, "one CTA's shared memory");
+    if (npol == 2)
+        return a.nsig <= 32 ? launch_xsplit_n<32, 2>(a, cpx, d_err, nsm, st) : launch_xsplit_n<64, 2>(a, cpx, d_err, nsm, st);
+    return a.nsig <= 32 ? launch_xsplit_n<32, 1>(a, cpx, d_err, nsm, st) : launch_xsplit_n<64, 1>(a, cpx, d_err, nsm, st);
+}
+
+}  // namespace fx

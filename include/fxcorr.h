@@ -43,11 +43,13 @@ extern "C" {
 #define FXC_ERR_TIMEOUT      -6   /* a bounded device-side wait expired; that call's result is invalid */
 
 /* X-stage arithmetic */
-#define FXC_X_PLAIN_FP32 0        /* FP32 CUDA-core cross-multiply-accumulate */
+#define FXC_X_PLAIN_FP32 0        /* FP32 cross-multiply-accumulate: on the FP32 units or, with up to 64 signals and
+                                     enough channels, on the tensor cores (each FP32 value as two FP16 ones, FP32
+                                     sums flushed every 16 FFTs: FP32-grade results, chosen by geometry) */
 #define FXC_X_TC_FP16    1        /* tcgen05 tensor cores, FP16 inputs, FP32 accumulation (on the FFT F
-                                     stage with <= 64 signals the F stage writes FP32 spectra and the X
-                                     stage rounds them to FP16 itself; FXC_TC_SPECTRA=f16 in the
-                                     environment at context creation keeps the F stage's FP16 layout) */
+                                     stage with <= 64 signals the X stage turns the FP16 spectra itself;
+                                     FXC_TC_SPECTRA=f16 in the environment at context creation has them
+                                     turned in memory, as beyond 64 signals) */
 #define FXC_X_TC_FP8     2        /* tcgen05 tensor cores, FP8-E4M3 inputs scaled per antenna, polarisation and
                                      channel by 448/absmax over each spectra chunk, FP32 accumulation */
 
@@ -227,9 +229,9 @@ int fxc_correlate_noalloc(const fxc_config* cfg, const uint8_t* d_data, size_t p
  * one CUDA graph of the whole sequence.  FXC_ERR_UNSUPPORTED for the FP8 form,
  * input windows, 8-bit complex input and the tensor-core F stages.
  * No counterpart in the reference (one job per run).
- * fxc_batch_autotune times the FFT block size (8/16/32 FFTs per CTA) of every
- * F group and the tile variant of every X group on the uploaded data, keeps the
- * fastest, and zeroes the accumulators; with the environment variable
+ * fxc_batch_autotune times the FFT block size (8/16/32 FFTs per task) of every
+ * F group and the tile variant of every X group (the jobs on the FP32 units) on the uploaded data, keeps
+ * the fastest, and zeroes the accumulators; with the environment variable
  * FXC_PLAN_CACHE naming a file, chosen plans are appended to it and read back by
  * later fxc_batch_create calls. */
 typedef struct fxc_batch fxc_batch;
@@ -253,9 +255,11 @@ int fxc_batch_use_graph(fxc_batch* b, int enable);
  * builds the task tables if needed; < 0 on error */
 int fxc_batch_launch_count(fxc_batch* b);
 
-/* Launch plan of a context: FFTs per F-stage CTA (8, 16 or 32) and plain X tile variant (0 or 1).
+/* Launch plan of a context: FFTs per F-stage task of a batch (8, 16 or 32) and tile variant of the
+ * plain X stage on the FP32 units (0 or 1).
  * Defaults 16 / 0, or the entries of the plan-cache file named by the environment variable
- * FXC_PLAN_CACHE when the context is created.  Plans change speed only, never results. */
+ * FXC_PLAN_CACHE when the context is created.  Plans change speed only, never results; a context alone draws its
+ * FFTs from a counter, whatever the first number. */
 int fxc_set_plan(fxc_ctx* ctx, int fft_block, int x_variant);
 int fxc_get_plan(fxc_ctx* ctx, int* fft_block, int* x_variant);
 /* Times every plan on the context's current input and delay model (at least one earlier
@@ -320,6 +324,10 @@ int fxc_debug_expire_wait_tc(fxc_ctx* ctx);
  * *tseg segments of *tlen slots (1 and T: no cut).  Host arithmetic only; the library takes
  * the occupancy of its default tile variant on the context's GPU for `slots`. */
 int fxc_debug_xplain_segments(long long ctas, long long slots, int T, int* tseg, int* tlen);
+
+/* 1 if the plain form of this geometry (signals = antennas x polarisations) runs its X stage on the tensor cores
+ * (FP32 values as FP16 pairs, FP32 sums), 0 if on the FP32 units.  Host arithmetic only. */
+int fxc_debug_xsplit_pays(int nsig, int nchan, int nsb, int numffts, int nsm);
 
 #if defined(__GNUC__)
 #pragma GCC visibility pop
