@@ -47,8 +47,20 @@
 // while the slot's first thread describes pair i + 2, copies its bytes and fetches the delay
 // entries of pair i + 3.
 //
+// Real samples at 1024 and 2048 points (PPlan::R32) take a plan with one exchange instead of two: 32 points a thread
+// (32 x 32; 64 x 32 with two threads to a set of 64 samples, each of which decodes all of them and forms its half of
+// stage 0's outputs), 290 wavefronts per 1024 samples instead of 400 to 455, one barrier fewer, coalesced runs of 32
+// channels.  It costs 184 registers, so 8 warps per SM: too few to hide a pair's preparation, which a helper warp
+// per slot does instead -- descriptors in registers, samples straight from global memory, factor
+// tables three FP64 chains abreast -- and meets the slot's threads at two barriers per pair:
+//   helper:  words and factors of pair i + 1                | expansion, pass 0 twiddles of i + 1, entries of i + 2
+//   others:  stage 0, pass 0 of pair i                      | exchange, pass 1, correction, store
+// 23 antennas x 3 subbands x 2777 FFTs of 1024 points: 0.459 -> 0.351 ms; 64 antennas x 8 subbands x 31250 FFTs of
+// 2048 points: 72 -> 65.5 ms (power-limited: 1.85 GHz).  Without the helper 0.450 and 67.9.  At 4096 points this plan
+// needs a radix 2 over lanes (64 shuffles a thread) or half the warps and gains nothing.
+//
 // Measured (B200, against one scalar FFT per slot, fx_fscalar.cuh with FP32 spectra): 64 antennas x 8 subbands
-// x 31250 FFTs of 2048 points, one polarisation: 89.7 -> 70.6 ms (464 Gsamp/s); 16 antennas x 2
+// x 31250 FFTs of 2048 points, one polarisation: 89.7 -> 70.6 ms (464 Gsamp/s; now R32); 16 antennas x 2
 // polarisations x 4 subbands x 31250 FFTs of 4096 points: 47.1 -> 32.8 ms (499 Gsamp/s).
 #pragma once
 
@@ -191,27 +203,36 @@ template <int F, int NPOL, bool CPX>
 struct PPlan {
     using P = FPlan<F, CPX>;
     static constexpr int C = P::C;
-    static constexpr int NT = F / 16;
+    // real samples at 1024 and 2048 points: one exchange, 32 points per thread, H0 threads share a sample
+    static constexpr bool R32 = !CPX && (F == 1024 || F == 2048);
+    static constexpr int H0 = R32 && F == 2048 ? 2 : 1;
+    static constexpr int NT = R32 ? F / 32 : F / 16;
     static constexpr int LOGF = ilog2c(F);
     static constexpr int LOGS = ilog2c(P::S);
     static constexpr int NPASS = P::NPASS;
     static constexpr int LASTR = P::LASTR;
     // slots of a CTA: 256 threads (complex samples at 256 points: 14 slots, what half an SM's shared memory holds)
-    static constexpr int NSLOT = CPX && F == 256 ? 14 : P::NSLOT;
-    static constexpr int NTHREADS = NT * NSLOT;
-    static constexpr int MINB = P::MINB;
-    static constexpr int NE = CPX ? 16 : 8;                // channels a thread stores
+    static constexpr int NSLOT = R32 ? 256 / NT : CPX && F == 256 ? 14 : P::NSLOT;
+    // R32: a helper warp per slot, which prepares pairs; registers of compute and helper threads (their sum is what the
+    // block is launched with, 168 or 128 a thread; splits by 8 either way measured 1 to 9 % slower)
+    static constexpr int NCOMP = NT * NSLOT;
+    static constexpr int NTHREADS = NCOMP + (R32 ? 32 * NSLOT : 0);
+    static constexpr int PN = R32 ? 32 : NT;               // threads that prepare a slot's pairs
+    static constexpr int R_COMP = 184, R_HELP = F == 2048 ? 136 : 72;
+    static constexpr int MINB = R32 ? 1 : P::MINB;
+    static constexpr int NE = CPX || R32 ? 16 : 8;         // channels a thread stores
     static constexpr int HI = NT / 16;
     static constexpr int NTAB = LOGF + 16 + HI + NE;       // rho, E low, E high, G
     static constexpr int NLANE = NPOL == 2 ? 1 : 2;        // delay entries of a pair
     static constexpr int R2 = NPASS == 2 ? 0 : NPASS == 3 ? LASTR : 16;   // radix of pass 2
-    static constexpr int D2 = R2 / 2;
-    static constexpr bool W1TAB = F > (CPX ? 1024 : 512);  // pass 1 twiddles per pair in a table
+    static constexpr int D2 = R32 ? 0 : R2 / 2;
+    static constexpr bool W1TAB = !R32 && F > (CPX ? 1024 : 512);  // pass 1 twiddles per pair in a table
     // factor tables kept: those of pair i + 1 are written before the barrier that ends pair i - 1's
     // reads, except where a slot is half a warp or (complex input) they are written after it
-    static constexpr int NTABS = CPX || NT < 32 ? 2 : 4;
-    static constexpr int BUF = F + F / 16;                 // padded exchange buffer (float4)
-    static constexpr int INB = fstage_inb<F, NPOL, CPX>() + 16;   // one window (and the read past its last word)
+    static constexpr int NTABS = R32 || CPX || NT < 32 ? 2 : 4;
+    static constexpr int BUF = R32 ? F + F / 32 : F + F / 16;   // padded exchange buffer (float4)
+    // one window (and the read past its last word); R32 stages none
+    static constexpr int INB = R32 ? 16 : fstage_inb<F, NPOL, CPX>() + 16;
 };
 
 // What the slot's threads need of a pair.
@@ -235,9 +256,9 @@ struct PairSlot {              // shared memory of one slot
     float4 buf[P::BUF];
     using Fe = typename Fac<NPOL>::T;
     Fe tab[P::NTABS][P::NTAB]; // by pair number
-    Fe w0[8];                  // pass 0: 1 .. 7 of the twiddle order
+    Fe w0[P::R32 ? 16 * P::H0 : 8];   // pass 0: 1 .. 7 of the twiddle order (R32: 16 per stage 0 output)
     Fe w1[P::W1TAB ? 2 : 1][P::W1TAB ? 128 : 2];   // by pair parity
-    DelayEntry dent[4][2];
+    DelayEntry dent[P::R32 ? 1 : 4][2];
     PairLoc loc[4];
     alignas(16) uint8_t inb[P::NLANE][P::INB];
     alignas(16) uint8_t xs[CPX ? 16 : F];
@@ -249,16 +270,17 @@ template <int F, int NPOL, bool CPX>
 struct PairSmem {
     using P = PPlan<F, NPOL, CPX>;
     PairSlot<F, NPOL, CPX> slot[P::NSLOT];
-    float4 w1c[128];           // constant part of pass 1's twiddles [8][16] and its rounding
+    float4 w1c[P::R32 ? 1 : 128];      // constant part of pass 1's twiddles [8][16] and its rounding
+    float2 wbc[P::R32 ? 16 * P::NT : 1];               // R32: constant part of pass 1's twiddles [16][NT]
     float2 w2c[P::D2 ? P::D2 * 256 : 2];               // constant part of pass 2's twiddles [D2][256]
     float2 lut[16];            // levels of codes (A, B)
-    float4 w0c[8];             // the same of pass 0
+    float4 w0c[P::R32 ? 16 * P::H0 : 8];               // as w1c, of pass 0
 };
 
 template <int NT>
 __device__ __forceinline__ void pair_sync(int slot)
 {
-    if constexpr (NT >= 32) {
+    if constexpr (NT > 32) {
         asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "r"(NT) : "memory");
     } else {
         __syncwarp();
@@ -292,7 +314,7 @@ __device__ __forceinline__ double2 cospi_d(double x)
 // what its rounding to FP32 left
 __device__ __forceinline__ float4 pass_w(int d, int jm, int NS)
 {
-    const int q = d == 0 ? 0 : d == 1 ? 1 : d < 4 ? 2 : 3;
+    const int q = d == 0 ? 0 : 32 - __clz(d);
     const int kp = d - (q == 0 ? 0 : 1 << (q - 1));
     const double inv = __hiloint2double((1023 - (31 - __clz(NS)) - (q + 1)) << 20, 0);   // 1 / (NS 2^(q+1))
     const double2 w = cospi_d(-2.0 * (jm + NS * kp) * inv);
@@ -300,35 +322,40 @@ __device__ __forceinline__ float4 pass_w(int d, int jm, int NS)
     return make_float4(x, y, __double2float_rn(w.x - (double)x), __double2float_rn(w.y - (double)y));
 }
 
-// Table entry e of one lane: rho - 1 of stage e, then E[t & 15], E[t >> 4], G.
+// Table entry e of one lane: rho - 1 of stage e, then E[t & 15], E[t >> 4], G.  Its angle in half-turns (of one
+// form for all entries: a warp's threads don't part):
 template <int F, int NPOL, bool CPX>
-__device__ __forceinline__ float2 pair_entry(int e, const DelayEntry& d, double lo, double chalf)
+__device__ __forceinline__ double pair_angle(int e, double da, double db, double frac, double lo, double chalf)
 {
     using P = PPlan<F, NPOL, CPX>;
     constexpr int LOGSTRIDE = P::LOGF - P::LOGS;
-    if (e < P::LOGF) {
-        // kernel.c:145, 434-470: bit b of n weighs 2^b / F below S, 2^b / S steps of stride / F above
-        const int b = P::LOGF - 1 - e;
-        const int ex = (b < P::LOGS ? b : b - P::LOGS + LOGSTRIDE) - P::LOGF;
-        const double weight = __hiloint2double((1023 + ex) << 20, 0);
-        const double ph = dmul(dmul(weight, d.a), lo);
-        const double2 r = cospi_d(-2.0 * dsub(ph, rint(ph)));
-        return make_float2(__double2float_rn(r.x - 1.0), __double2float_rn(r.y));
-    }
+    // the FFT's constant phase, kernel.c:434-466: lo b', b' = b - (int)b, and the LO's fraction
+    const double whole = trunc(db);
+    double ph = dmul(dsub(db, whole), lo);
+    const double lofrac = dsub(lo, trunc(lo));
+    if (lofrac > 1e-11) ph = dadd(ph, dmul(lofrac, whole));   // kernel.c:39
+    ph = 2.0 * dsub(ph, rint(ph));
+    // kernel.c:145, 434-470: bit b of n weighs 2^b / F below S, 2^b / S steps of stride / F above
+    const bool rho = e < P::LOGF;
+    const int b = P::LOGF - 1 - e;
+    const int ex = (b < P::LOGS ? b : b - P::LOGS + LOGSTRIDE) - P::LOGF;
     const int k = e - P::LOGF;
     const int c = k < 16 ? k : k < 16 + P::HI ? 16 * (k - 16) : P::NT * (k - 16 - P::HI);
-    double x = dmul(dmul((double)c, chalf), d.frac);
-    if (k >= 16 + P::HI) {
-        // the FFT's constant phase, kernel.c:434-466: lo b', b' = b - (int)b, and the LO's fraction
-        const double whole = trunc(d.b);
-        double ph = dmul(dsub(d.b, whole), lo);
-        const double lofrac = dsub(lo, trunc(lo));
-        if (lofrac > 1e-11) ph = dadd(ph, dmul(lofrac, whole));   // kernel.c:39
-        x = dsub(x, 2.0 * dsub(ph, rint(ph)));
-    }
-    x = dsub(x, 2.0 * rint(0.5 * x));
-    const double2 r = cospi_d(x);
-    const float sg = __popc(c) & 1 ? -1.f : 1.f;   // sign of the FMA-form butterflies
+    const double w = rho ? __hiloint2double((1023 + ex) << 20, 0) : (double)c;
+    double x = dmul(dmul(w, rho ? da : chalf), rho ? lo : frac);
+    x = rho ? -2.0 * x : dsub(x, k >= 16 + P::HI ? ph : 0.0);
+    return dsub(x, 2.0 * rint(0.5 * x));
+}
+// and its value, of (cos, sin) of that angle
+template <int F, int NPOL, bool CPX>
+__device__ __forceinline__ float2 pair_entry(int e, double2 r)
+{
+    using P = PPlan<F, NPOL, CPX>;
+    if (e < P::LOGF) return make_float2(__double2float_rn(r.x - 1.0), __double2float_rn(r.y));
+    const int k = e - P::LOGF;
+    const int c = k < 16 ? k : k < 16 + P::HI ? 16 * (k - 16) : P::NT * (k - 16 - P::HI);
+    // sign of the FMA-form butterflies (two threads' stage 0 outputs are plain sums)
+    const float sg = __popc(c & ~(P::H0 - 1)) & 1 ? -1.f : 1.f;
     return make_float2(sg * __double2float_rn(r.x), sg * __double2float_rn(r.y));
 }
 
@@ -337,8 +364,11 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
 {
     using P = PPlan<F, NPOL, CPX>;
     constexpr int NT = P::NT;
-    const int slot = threadIdx.x / NT;
-    const int t = threadIdx.x - slot * NT;
+    constexpr int PN = P::PN;
+    const bool helper = P::R32 && threadIdx.x >= P::NCOMP;
+    const int slot = helper ? (threadIdx.x - P::NCOMP) / 32 : threadIdx.x / NT;
+    const int t = helper ? threadIdx.x & 31 : threadIdx.x - slot * NT;
+    const bool lead = t == 0 && helper == P::R32;   // of the threads that draw the slot's pairs
     PairSlot<F, NPOL, CPX>& s = sm.slot[slot];
     using Fe = typename Fac<NPOL>::T;
     auto fac = [](Fe f) { return Fac<NPOL>::get(f); };
@@ -362,13 +392,16 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
     };
     const bool drawn = nitem > 3 * nwork * PT;   // otherwise no slot gets a fourth pair
 
+    // stage of twiddle d (order of wfirst)
+    auto stage_of = [](int d) { return d == 0 ? 0 : 32 - __clz(d); };
+
     // ---- slot's first thread: descriptor and delay entries of pair i, then its bytes
     auto fetch = [&](int i) {
         PairLoc& L = s.loc[i & 3];
         L.has = L.wr = L.valid = 0;
         L.end = ticket * PT >= nitem;
         const int g = ticket * PT + slot % PT;
-        if (!L.end) ticket = i < 2 || !drawn ? ticket + nwork : draw();   // needed one pair later
+        if (!L.end && !P::R32) ticket = i < 2 || !drawn ? ticket + nwork : draw();   // needed one pair later
         if (g < nitem) {
             locate(g, L);
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32a(&L.lo)), "l"(L.plo) : "memory");
@@ -389,14 +422,13 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
     // (kernel.c:402-409: F NPOL / 4 bytes and the read-ahead byte, or 2 NPOL bytes per complex
     // sample) begins at the 16-byte boundary at or below the first byte
     constexpr int SB = CPX ? 16 * NPOL : 2 * NPOL;   // bits per sample
-    auto describe = [&](int i) {
-        PairLoc& L = s.loc[i & 3];
+    auto describe = [&](PairLoc& L, const DelayEntry* dent) {
         int valid = 0;
 #pragma unroll
         for (int l = 0; l < P::NLANE; l++) {
             L.bit[l] = 0;
             if ((L.has >> l) & 1) {
-                const DelayEntry& d = s.dent[i & 3][l];
+                const DelayEntry& d = dent[l];
                 if (d.valid) {
                     valid |= 1 << l;
                     const long long bit = (long long)d.offset * SB;
@@ -408,8 +440,7 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
         L.valid = valid;
     };
     // the windows of pair i: whole 16-byte vectors by the bulk-copy engine
-    auto copy = [&](int i) {
-        const PairLoc& L = s.loc[i & 3];
+    auto copy = [&](const PairLoc& L) {
         if (!L.valid) return;
         uint32_t bytes[P::NLANE], total = 0;
 #pragma unroll
@@ -417,7 +448,6 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
             bytes[l] = (L.valid >> l) & 1 ? 16u * ((F * SB / 8 + (CPX ? 0 : 1) + (L.bit[l] >> 3) + 15) >> 4) : 0u;
             total += bytes[l];
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32a(&s.bar)), "r"(total)
                      : "memory");
 #pragma unroll
@@ -433,18 +463,35 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
             }
     };
     // factor tables of pair i, by the slot's last threads (the first one is busy with descriptors)
-    auto factors = [&](int i) {
-        const PairLoc& L = s.loc[i & 3];
+    auto factors = [&](int i, const PairLoc& L, const DelayEntry* dent) {
         float* tab = reinterpret_cast<float*>(s.tab[i & (P::NTABS - 1)]);   // single polarisation: lanes interleaved
-        for (int u = NT - 1 - t; u < P::NTAB * P::NLANE; u += NT) {
-            const int e = u / P::NLANE, l = u % P::NLANE;
-            float2 r = make_float2(0.f, 0.f);   // an invalid lane's spectrum is zero
-            if ((L.valid >> l) & 1) r = pair_entry<F, NPOL, CPX>(e, s.dent[i & 3][l], L.lo, L.chalf);
-            if constexpr (NPOL == 2) {
-                s.tab[i & (P::NTABS - 1)][e] = r;
-            } else {
-                tab[4 * e + l] = r.x;
-                tab[4 * e + 2 + l] = r.y;
+        // (a helper's few rounds side by side: each is a chain of some thirty FP64 instructions)
+        constexpr int N = P::NTAB * P::NLANE, NR = P::R32 ? (N + PN - 1) / PN : 1;
+        for (int u0 = PN - 1 - t; u0 < N; u0 += NR * PN) {
+            double x[NR];
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const int u = u0 + r * PN, e = u / P::NLANE, l = u % P::NLANE;
+                constexpr int B = P::NLANE - 1;
+                const double da = l ? dent[B].a : dent[0].a, db = l ? dent[B].b : dent[0].b;
+                const double df = l ? dent[B].frac : dent[0].frac;
+                x[r] = u < N && ((L.valid >> l) & 1) ? pair_angle<F, NPOL, CPX>(e, da, db, df, L.lo, L.chalf) : 0.0;
+            }
+            double2 cs[NR];
+#pragma unroll
+            for (int r = 0; r < NR; r++) cs[r] = cospi_d(x[r]);
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const int u = u0 + r * PN, e = u / P::NLANE, l = u % P::NLANE;
+                if (u >= N) break;
+                float2 v = make_float2(0.f, 0.f);   // an invalid lane's spectrum is zero
+                if ((L.valid >> l) & 1) v = pair_entry<F, NPOL, CPX>(e, cs[r]);
+                if constexpr (NPOL == 2) {
+                    s.tab[i & (P::NTABS - 1)][e] = v;
+                } else {
+                    tab[4 * e + l] = v.x;
+                    tab[4 * e + 2 + l] = v.y;
+                }
             }
         }
     };
@@ -460,28 +507,46 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
             phase ^= 1;
         }
     };
+    // at the end of the slot's pairs
+    auto finish = [&] {
+        // after an expired wait the copy may still land: wait for it once more (bounded) so it cannot
+        // write into an exited CTA's shared memory
+        if (!P::R32 && expired) stg_wait(&s.bar, phase ^ 1);
+        if (drawn && lead && slot % PT == 0) {
+            __threadfence();   // this worker's draws come before its count
+            if (atomicAdd(ctr + 1, 1) == nwork - 1) {
+                ctr[0] = 0;
+                ctr[1] = 0;
+            }
+        }
+    };
     // 2-bit real samples of pair i: one byte per sample pair, the offset of its levels in the table.  The
     // words of 16 samples are permuted so that pass 0's reads, NT / 16 samples apart, hit distinct banks.
-    constexpr int SWZ = NT == 512 ? 3 : NT == 256 ? 1 : 0;   // bits of n >> 7 taken into the word number
-    auto expand = [&](int i) {
-        const PairLoc& L = s.loc[i & 3];
+    constexpr int SWZ = P::R32 ? 0 : NT == 512 ? 3 : NT == 256 ? 1 : 0;   // bits of n >> 7 taken into the word number
+    struct Words { uint32_t w[NPOL == 2 ? 3 : 4]; };
+    auto load16 = [&](const PairLoc& L, int t) {   // the words with samples 16 t .. 16 t + 15
+        Words a;
+#pragma unroll
+        for (int l = 0; l < P::NLANE; l++) {
+            const uint32_t* wp = reinterpret_cast<const uint32_t*>(s.inb[l]) + NPOL * t + (L.bit[l] >> 5);
+#pragma unroll
+            for (int k = 0; k < NPOL + 1; k++) a.w[2 * l + k] = wp[k];
+        }
+        return a;
+    };
+    auto expand16 = [&](const int (&sh)[P::NLANE], int t, const Words& a) {   // sh: the first one's bit in its word
         uint32_t nib[2];   // 8 samples each: codes (A, B) of sample k in bits 4 k .. 4 k + 3
         if constexpr (NPOL == 2) {
-            const int bit = L.bit[0];
-            const uint32_t* wp = reinterpret_cast<const uint32_t*>(s.inb[0]) + 2 * t + (bit >> 5);
-            const uint32_t a0 = wp[0], a1 = wp[1], a2 = wp[2];
-            nib[0] = __funnelshift_r(a0, a1, bit & 31);
-            nib[1] = __funnelshift_r(a1, a2, bit & 31);
+            nib[0] = __funnelshift_r(a.w[0], a.w[1], sh[0]);
+            nib[1] = __funnelshift_r(a.w[1], a.w[2], sh[0]);
         } else {
             uint32_t sp[2][2];
 #pragma unroll
             for (int l = 0; l < 2; l++) {
-                const int bit = L.bit[l];
-                const uint32_t* wp = reinterpret_cast<const uint32_t*>(s.inb[l]) + t + (bit >> 5);
-                const uint32_t a = __funnelshift_r(wp[0], wp[1], bit & 31);
+                const uint32_t b = __funnelshift_r(a.w[2 * l], a.w[2 * l + 1], sh[l]);
 #pragma unroll
                 for (int h = 0; h < 2; h++) {   // 2-bit groups of a half word to every second group
-                    uint32_t x = h ? a >> 16 : a & 0xFFFFu;
+                    uint32_t x = h ? b >> 16 : b & 0xFFFFu;
                     x = (x | (x << 8)) & 0x00FF00FFu;
                     x = (x | (x << 4)) & 0x0F0F0F0Fu;
                     sp[l][h] = (x | (x << 2)) & 0x33333333u;
@@ -510,10 +575,24 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
             }
         *reinterpret_cast<uint4*>(s.xs + 16 * t) = make_uint4(o[0], o[1], o[2], o[3]);
     };
+    constexpr int NG = P::R32 ? F / 512 : 1;
+    auto expand_w = [&](const PairLoc& L, const Words (&a)[NG]) {
+        int sh[P::NLANE];
+#pragma unroll
+        for (int l = 0; l < P::NLANE; l++) sh[l] = L.bit[l] & 31;
+#pragma unroll
+        for (int g = 0; g < NG; g++) expand16(sh, t + g * PN, a[g]);
+    };
+    auto expand = [&](const PairLoc& L) {   // from the staged bytes
+        const Words a[NG] = {load16(L, t)};
+        expand_w(L, a);
+    };
     // twiddles of passes 0 and 1 with pair i's rho
     auto twiddles = [&](int i) {
         const Fe* tab = s.tab[i & (P::NTABS - 1)];
-        if (t < 8 && t > 0) {
+        if constexpr (P::R32) {
+            for (int e = t; e < 16 * P::H0; e += PN) s.w0[e] = mul_hl(tab[P::H0 - 1 + stage_of(e & 15)], sm.w0c[e]);
+        } else if (t < 8 && t > 0) {
             const int q = t == 1 ? 1 : t < 4 ? 2 : 3;
             s.w0[t] = mul_hl(tab[q], sm.w0c[t]);
         }
@@ -526,40 +605,131 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
         }
     };
 
-    if (t == 0) {
+    // R32: the helper's lanes hold the next pair's descriptor in registers, all the same (a chain of loads from shared
+    // memory takes 300 cycles a link beside the other warps), and leave the other threads what they store by
+    PairLoc nxt;
+    DelayEntry dnxt[P::NLANE];
+    auto load = [&](int i, int k) {   // pair i of the slot: ticket k
+        nxt.has = nxt.wr = 0;
+        nxt.end = k >= nitem;
+        if (!nxt.end) {
+            locate(k, nxt);
+            nxt.lo = __ldg(nxt.plo);
+        }
+#pragma unroll
+        for (int l = 0; l < P::NLANE; l++) {
+            dnxt[l].offset = dnxt[l].valid = 0;
+            if ((nxt.has >> l) & 1) {
+                const int4* src = reinterpret_cast<const int4*>(nxt.d + l);
+                reinterpret_cast<int4*>(&dnxt[l])[0] = __ldg(src);
+                reinterpret_cast<int4*>(&dnxt[l])[1] = __ldg(src + 1);
+            }
+        }
+        if (t == 0) {
+            PairLoc& S = s.loc[i & 3];
+            S.out = nxt.out;
+            S.out_b = nxt.out_b;
+            S.wr = nxt.wr;
+            S.end = nxt.end;
+        }
+    };
+    // the words with the samples that a lane expands, from global memory: those alone that hold needed bits
+    auto words = [&](Words (&a)[NG]) {
+#pragma unroll
+        for (int l = 0; l < P::NLANE; l++) {
+            const long long bit = (long long)dnxt[l].offset * SB;
+            nxt.bit[l] = (int)bit & 31;
+            const uint32_t* wp = reinterpret_cast<const uint32_t*>(nxt.row) + (bit >> 5) + NPOL * t;
+            const bool on = dnxt[l].valid;
+#pragma unroll
+            for (int g = 0; g < NG; g++)
+#pragma unroll
+                for (int k = 0; k < NPOL + 1; k++) {
+                    uint32_t w = 0;   // (volatile: here, not where the word is used)
+                    if (on && (k < NPOL || nxt.bit[l]))
+                        asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(w) : "l"(wp + 32 * NPOL * g + k));
+                    a[g].w[2 * l + k] = w;
+                }
+        }
+        nxt.valid = 0;
+#pragma unroll
+        for (int l = 0; l < P::NLANE; l++) nxt.valid |= dnxt[l].valid ? 1 << l : 0;
+    };
+    if constexpr (P::R32) {
+        if (helper) load(0, ticket);
+    } else if (t == 0) {
         fetch(0);
         fetch(1);
     }
     // ---- constant tables of the CTA
-    for (int e = threadIdx.x; e < 128; e += P::NTHREADS) sm.w1c[e] = pass_w(e >> 4, e & 15, 16);
+    if constexpr (P::R32) {
+        for (int e = threadIdx.x; e < 16 * NT; e += P::NTHREADS) {
+            const float4 w = pass_w(e / NT, e % NT, 32 * P::H0);
+            sm.wbc[e] = make_float2(w.x, w.y);
+        }
+    } else {
+        for (int e = threadIdx.x; e < 128; e += P::NTHREADS) sm.w1c[e] = pass_w(e >> 4, e & 15, 16);
+    }
     for (int e = threadIdx.x; e < P::D2 * 256; e += P::NTHREADS) {
         const float4 w = pass_w(e >> 8, e & 255, 256);
         sm.w2c[e] = make_float2(w.x, w.y);
     }
     if (threadIdx.x < 16) sm.lut[threadIdx.x] = make_float2(level2bit(threadIdx.x & 3), level2bit(threadIdx.x >> 2));
-    if (threadIdx.x < 8) sm.w0c[threadIdx.x] = pass_w(threadIdx.x, 0, 1);
-    if (t == 0) {
+    if (threadIdx.x < (P::R32 ? 16 * P::H0 : 8)) sm.w0c[threadIdx.x] = pass_w(threadIdx.x & 15, threadIdx.x >> 4, P::H0);
+    if (!P::R32 && t == 0) {
         stg_bar_init(&s.bar);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (t == 0) {
+    if (!P::R32 && t == 0) {
         entries_wait();
-        describe(0);
-        copy(0);
-        describe(1);
+        describe(s.loc[0], s.dent[0]);
+        copy(s.loc[0]);
+        describe(s.loc[1], s.dent[1]);
         fetch(2);
     }
     __syncthreads();
-    factors(0);
+    // R32: the helper meets the slot's threads before pass 0 (a pair is prepared) and after it (the samples and the
+    // twiddles of pass 0 are free)
+    auto meet = [&] { asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "r"(NT + 32) : "memory"); };
+    if constexpr (P::R32) {
+        if (helper) {
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P::R_HELP));
+            const bool any = !nxt.end;
+            int ahead = 0;   // lane 1: the ticket of pair i + 3, drawn one pair earlier
+            for (int i = -1; !nxt.end; i++) {   // nxt is pair i + 1
+                Words a[NG];
+                if (i >= 0) meet();
+                words(a);
+                factors(i + 1, nxt, dnxt);
+                if (i >= 0) meet();
+                __syncwarp();
+                expand_w(nxt, a);
+                twiddles(i + 1);
+                const int k = __shfl_sync(0xffffffffu, ahead, 1);
+                if (drawn && i >= 0 && t == 1) ahead = 3 * nwork + atomicAdd(ctr, 1);
+                load(i + 2, i < 1 || !drawn ? ticket + (i + 2) * nwork : k);
+            }
+            if (any) {   // the last pair
+                meet();
+                meet();
+            }
+            __syncwarp();   // lane 1's last draw comes before lane 0's fence
+            finish();
+            return;
+        }
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P::R_COMP));
+    } else {
+    factors(0, s.loc[0], s.dent[0]);
     pair_sync<NT>(slot);
     if constexpr (!CPX) {
         bytes_wait(s.loc[0]);
-        expand(0);
+        expand(s.loc[0]);
     }
     twiddles(0);
     pair_sync<NT>(slot);
     if constexpr (!CPX)
-        if (t == 0) copy(1);
+        if (t == 0) copy(s.loc[1]);
+    }
 
     const float4* buf_t = s.buf + padi(t);
     float4* row_t = s.buf + 272 * (t >> 4);   // exchange rows of the threads with this d0
@@ -571,7 +741,63 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
         const PairLoc& L = s.loc[i & 3];
         const bool more = !s.loc[(i + 1) & 3].end;
         const Fe* tab = s.tab[i & (P::NTABS - 1)];
-        c2 v[16];
+        c2 v[P::R32 ? 32 : 16];
+        auto next = [&] {
+            if (more) {
+                if constexpr (!CPX) {
+                    bytes_wait(s.loc[(i + 1) & 3]);
+                    expand(s.loc[(i + 1) & 3]);
+                }
+                twiddles(i + 1);
+            }
+            pair_sync<NT>(slot);
+            if constexpr (!CPX)
+                if (t == 0) copy(s.loc[(i + 2) & 3]);
+        };
+        if constexpr (P::R32) {
+            // ---- stage 0 on real samples (output h of two: x +- rho x'), stages 1 to 4 + H0 of thread tp's 32 H0
+            // samples, one of its H0 sets of 32 outputs k1 = h + H0 r
+            constexpr int G = NT / P::H0;
+            meet();
+            const int h = t / G, tp = t % G;
+            const c2 r0 = fac(Fac<NPOL>::rho(tab[0]));
+            const unsigned char* lut = reinterpret_cast<const unsigned char*>(sm.lut);
+            const uint8_t* xp = s.xs + tp;
+            auto level = [&](int n) { return *reinterpret_cast<const float2*>(lut + xp[n]); };
+            if constexpr (P::H0 == 2) {
+                const c2 rs = h ? c2{neg2(r0.x), neg2(r0.y)} : r0;
+#pragma unroll
+                for (int r = 0; r < 32; r++) {
+                    const float2 x = level(r * G), x1 = level(r * G + F / 2);
+                    v[r].x = __ffma2_rn(rs.x, x1, x);
+                    v[r].y = __fmul2_rn(rs.y, x1);
+                }
+                butterfly<32, 0, false>(v, [&](int d) { return fac(s.w0[16 * h + d]); });
+            } else {
+                const float2 m2 = make_float2(-2.f, -2.f);
+#pragma unroll
+                for (int r = 0; r < 16; r++) {
+                    const float2 x = level(r * G), x1 = level((r + 16) * G);
+                    v[r].x = __ffma2_rn(r0.x, x1, x);
+                    v[r].y = __fmul2_rn(r0.y, x1);
+                    v[r + 16].x = __ffma2_rn(x, m2, v[r].x);
+                    v[r + 16].y = v[r].y;
+                }
+                butterfly<32, 1, false>(v, [&](int d) { return fac(s.w0[d]); });
+            }
+            meet();
+            // ---- exchange: rows k1 of G + 1; pass 1 takes row t
+#pragma unroll
+            for (int r = 0; r < 32; r++) s.buf[(h + P::H0 * r) * (G + 1) + tp] = as_f4(v[bitrev(r, 5)]);
+            if constexpr (NT > 32) asm volatile("bar.sync %0, %1;" ::"r"(P::NSLOT + slot + 1), "n"(NT) : "memory");
+            else __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 32; r++) v[r] = as_c2(s.buf[t * (G + 1) + r]);
+            butterfly<32, 0, true>(v, [&](int d) {
+                return fac(Fac<NPOL>::mul(tab[4 + P::H0 + stage_of(d)], sm.wbc[NT * d + t]));
+            });
+        } else {
+        // (not indented: the plan with an exchange per pass)
         // ---- pass 0
         {
             const c2 r0 = fac(Fac<NPOL>::rho(tab[0]));
@@ -613,17 +839,17 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
             }
         }
         if constexpr (!CPX)
-            if (more) factors(i + 1);
+            if (more) factors(i + 1, s.loc[(i + 1) & 3], s.dent[(i + 1) & 3]);
         pair_sync<NT>(slot);   // the exchange buffer, the samples and the twiddles of pass 0 are free
         if (t == 0) {
             entries_wait();
-            describe(i + 2);
+            describe(s.loc[(i + 2) & 3], s.dent[(i + 2) & 3]);
             fetch(i + 3);
-            if constexpr (CPX) copy(i + 1);
+            if constexpr (CPX) copy(s.loc[(i + 1) & 3]);
         }
         // ---- exchange and pass 1
         if constexpr (CPX) {
-            if (more) factors(i + 1);
+            if (more) factors(i + 1, s.loc[(i + 1) & 3], s.dent[(i + 1) & 3]);
 #pragma unroll
             for (int r = 0; r < 16; r++) s.buf[17 * t + r] = as_f4(v[bitrev(r, 4)]);
             pair_sync<NT>(slot);
@@ -652,18 +878,6 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
 #pragma unroll
             for (int r = 0; r < 16; r++) row_t[17 * r + u] = as_f4(v[bitrev(r, 4)]);
         }
-        auto next = [&] {
-            if (more) {
-                if constexpr (!CPX) {
-                    bytes_wait(s.loc[(i + 1) & 3]);
-                    expand(i + 1);
-                }
-                twiddles(i + 1);
-            }
-            pair_sync<NT>(slot);
-            if constexpr (!CPX)
-                if (t == 0) copy(i + 2);
-        };
         if constexpr (P::NPASS > 2) next();
         // ---- pass 2
         constexpr int R2 = P::R2 ? P::R2 : 16;
@@ -705,9 +919,10 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
                 v[2 * (b + 4)] = lo;
             }
         }
+        }
         // ---- constant phase, fractional-sample correction and sign; store channels t + NT e
         {
-            constexpr int RL = P::LASTR, NBL = 16 / RL, ML = ilog2c(RL);
+            constexpr int RL = P::R32 ? 32 : P::LASTR, NBL = P::R32 ? 1 : 16 / RL, ML = ilog2c(RL);
             const Fe* El = tab + P::LOGF;
             const Fe* G = El + 16 + P::HI;
             float2 ea, eb;   // E of lanes A and B
@@ -753,16 +968,7 @@ __device__ __forceinline__ void pair_worker(PairSmem<F, NPOL, CPX>& sm, int nite
         }
         if constexpr (P::NPASS == 2) next();
     }
-    // after an expired wait the copy may still land: wait for it once more (bounded) so it cannot
-    // write into an exited CTA's shared memory
-    if (expired) stg_wait(&s.bar, phase ^ 1);
-    if (drawn && t == 0 && slot % PT == 0) {
-        __threadfence();   // this worker's draws come before its count
-        if (atomicAdd(ctr + 1, 1) == nwork - 1) {
-            ctr[0] = 0;
-            ctr[1] = 0;
-        }
-    }
+    if constexpr (!P::R32) finish();
 }
 
 // Pair p of (subband sb, antenna ant) from chunk slot tb0 on: both polarisations of slot tb0 + p, or
