@@ -359,9 +359,8 @@ def run_reference_arm(args):
 # DRAM bytes per input sample of the F-stage kernels (2048-point FFTs), dram__bytes_read.sum +
 # dram__bytes_write.sum from one ncu capture each on the 64-antenna x 1024-channel profiling case,
 # divided by the samples of that launch: key (fstage, F16 output)
-# (profiles/kernels_cfg2s_ncu_full.txt for k_fstage, profiles/k_ftc_cfg2s_ncu.txt for k_ftc,
-# profiles/k_ftc32_cfg2s_ncu.txt for k_ftc32).
-FSTAGE_DRAM_BYTES_PER_SAMPLE = {(1, True): 2.17, (1, False): 4.16, (2, True): 2.17, (3, True): 2.18}
+# (profiles/k_ftc_cfg2s_ncu.txt for k_ftc, profiles/k_ftc32_cfg2s_ncu.txt for k_ftc32; none of k_fpair).
+FSTAGE_DRAM_BYTES_PER_SAMPLE = {(2, True): 2.17, (3, True): 2.18}
 
 
 # form -> (fxc_config.xmode, fxc_config.fstage)
@@ -371,15 +370,16 @@ FORMS = {"plain": (0, 1),     # FXC_X_PLAIN_FP32, FXC_F_FFT32
          "tc32f": (1, 3),     # FXC_X_TC_FP16 on the FP32-grade tensor-core F stage (FXC_F_TC32), the headline
          "fp8": (2, 1)}       # FXC_X_TC_FP8 on the FP32 FFT F stage
 XMODES = {k: v[0] for k, v in FORMS.items()}
-DTYPES = {"plain": "f32 (FFT F stage and X stage on the CUDA cores)",
-          "tc": "f32 FFT F stage (CUDA cores), spectra cast to f16 for the tensor-core X stage, f32 accumulate",
+DTYPES = {"plain": "f32 (FFT F stage on the CUDA cores; X stage on the CUDA cores or, up to 64 signals, on f16 pairs "
+                   "of f32 values on the tensor cores, f32 accumulate)",
+          "tc": "f32 FFT F stage (CUDA cores), spectra stored as f16 for the tensor-core X stage, f32 accumulate",
           "tc16f": "f16 tensor-core F stage (k_ftc: f16 DFT matrices and intermediate), f16 X inputs, "
                    "f32 accumulate",
           "tc32f": "f32-grade tensor-core F stage (k_ftc32: f16 hi+lo operand pairs, three products per GEMM, "
                    "f32 accumulate), spectra cast to f16 for the tensor-core X stage, f32 accumulate",
           "fp8": "f32 FFT F stage (CUDA cores), spectra cast to e4m3 scaled per signal and channel for the "
                  "tensor-core X stage, f32 accumulate"}
-F_KERNELS = {1: "k_fstage (fused unpack/shift/fringe/FFT/frac-delay, FP32 radix-16 FFT on the CUDA cores)",
+F_KERNELS = {1: "k_fpair (fused unpack/shift/fringe/FFT/frac-delay, pairs of FFTs in packed FP32 on the CUDA cores)",
              2: "k_ftc (tcgen05 F stage: unpack/fringe, 32x64 DFT as two FP16 tensor-core GEMMs, twiddles, "
                 "frac-delay, F16 store)",
              3: "k_ftc32 (tcgen05 F stage, FP32-grade: 32x64 DFT as two tensor-core GEMMs on FP16 hi+lo pairs, "
@@ -401,9 +401,9 @@ def form_params(form, w):
 
 
 def spectra_f16(xmode, fstage, w):
-    """Whether the F stage writes the FP16 K-major spectra layout: the tensor-core forms, except the
-    FP16 form on the FFT F stage at up to 64 signals and a multiple of 4 channels, whose X stage
-    reads FP32 spectra and casts them itself (the library's rule, fx_api.cu ctx_create)."""
+    """Whether the X stage reads FP16 spectra in the K-major layout: the tensor-core forms, except the FP16
+    form on the FFT F stage at up to 64 signals and a multiple of 4 channels, whose X stage turns
+    channel-contiguous FP16 spectra itself (the library's rule, fx_api.cu ctx_create)."""
     import difx_tests_b200 as fx
     if xmode == fx.FXC_X_PLAIN_FP32:
         return False
@@ -526,7 +526,7 @@ def run_gpu_arm(args):
 
     # ---- roofline of the dominant kernel of the headline form (the F stage)
     hbm, tc_peak, peak_kind = peaks()
-    f16 = spectra_f16(xmode, fstage, w)
+    f16 = xmode != 0                 # the plain form's spectra are FP32
     spec_bpc = 4 if f16 else 8       # bytes per complex spectrum value written
     f_bytes = head["samples_per_launch"] * (0.25 + 0.5 * spec_bpc)
     f_gbs = f_bytes / (head["f_ms_launch"] / 1e3) / 1e9
@@ -541,7 +541,7 @@ def run_gpu_arm(args):
             "share": sm[1] / max(1e-9, sm.sum()),
             "note": ("latency-bound warp-specialised pipeline; HBM fraction shown for its algorithmic bytes"
                      if fstage in (2, 3) else
-                     "FP32 FFT is issue-bound on the CUDA cores; HBM fraction shown for its algorithmic bytes")}
+                     "FP32 FFT is bound by shared memory and the FP32 pipe; HBM fraction shown for its algorithmic bytes")}
 
     line = {
         "metric": METRIC, "value": head["value"], "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -950,9 +950,9 @@ def run_large_arm(args, emit=True, max_windows=None):
         "x_stage": {"tflops": tc["x_tflops"], "flop_per_step": tc["xflop"], "peak_tflops": tc_peak,
                     "frac": tc["x_tflops"] / tc_peak,
                     "note": "algorithmic Hermitian flops; 128x128 block pairs compute 12% more"},
-        "roofline": {"kernel": "k_fstage", "bound": "hbm", "achieved": f_gbs, "peak": hbm, "unit": "GB/s",
+        "roofline": {"kernel": "k_fpair", "bound": "hbm", "achieved": f_gbs, "peak": hbm, "unit": "GB/s",
                      "frac": f_gbs / hbm, "traffic": None, "peak_source": peak_kind + " (MEASURED_PEAKS.json)",
-                     "note": "F stage is FP32-issue-bound"},
+                     "note": "F stage is bound by shared memory and the FP32 pipe"},
         "clocks": tc["clocks"],
         "gpu_launches": int(tc["launches"].sum()),
         "plain": {"value": plain["value"], "unit": UNIT, "ms": plain["ms"],
