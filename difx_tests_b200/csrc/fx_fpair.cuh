@@ -61,7 +61,7 @@
 //
 // Measured (B200, against one scalar FFT per slot, fx_fscalar.cuh with FP32 spectra): 64 antennas x 8 subbands
 // x 31250 FFTs of 2048 points, one polarisation: 89.7 -> 70.6 ms (464 Gsamp/s; now R32); 16 antennas x 2
-// polarisations x 4 subbands x 31250 FFTs of 4096 points: 47.1 -> 32.8 ms (499 Gsamp/s).
+// polarisations x 4 subbands x 31250 FFTs of 4096 points: 47.1 -> 32.3 ms (507 Gsamp/s).
 #pragma once
 
 #include "fx_fstage.cuh"
