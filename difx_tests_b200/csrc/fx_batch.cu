@@ -176,7 +176,7 @@ static int build_tables(fxc_batch* b)
                 for (int sb = 0; sb < c->cfg.nsubband; sb++)
                     for (int c0 = 0; c0 < c->cfg.nchan; c0 += cg)
                         for (int s = 0; s < nseg; s++) tasks.push_back(make_int4(r * J + j, sb, c0, s));
-                if (nseg > 1) segd.push_back(j);
+                if (xj.tseg > 1) segd.push_back(j);   // its CTAs write partials, be it one segment in a short last chunk
             }
             if (tasks.size() > off) b->launches.push_back({kXGroup, g, off, (int)(tasks.size() - off), r});
             for (int j : segd) b->launches.push_back({kXReduce, j, 0, 0, r});
