@@ -260,6 +260,14 @@ __device__ __forceinline__ void umma_ss_acc(uint32_t tmem_d, uint64_t a, uint64_
                      ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc) : "memory");
 }
 
+// D = A B + 2^-S D (0 <= S <= 15)
+template <int S>
+__device__ __forceinline__ void umma_ss_scaled(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc)
+{
+    asm volatile("tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, 1, %4;"
+                 ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "n"(S) : "memory");
+}
+
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }

@@ -82,6 +82,8 @@ static_assert(128 * R_ISSUE + 32 * NCW * R_CAST + 32 * NEW * R_EPI <= NTHREADS *
 constexpr int EC = 16;                       // columns the epilogue reads at a time
 constexpr int TMEM_COLS = 512;               // two D: 4 x 64 columns each
 
+enum Input { kReal, kComplex, kComplexWide };   // 2-bit real samples; 8-bit complex, up to 1024 channels and beyond
+
 struct Smem {
     alignas(1024) uint8_t hi[NV * HT];
     alignas(1024) uint8_t lo[NV * LT];
@@ -132,7 +134,7 @@ __device__ __forceinline__ uint32_t h2(__half2 h) { return *reinterpret_cast<con
 
 // err: 1 a stage-full wait expired (cast or MMA); 2 a stage-free wait expired (producer or cast); 3 accumulator
 //      wait expired; 4 epilogue wait expired; 5 drain expired
-template <int NS, int NPOL, bool CPX>
+template <int NS, int NPOL, xsp::Input IN>
 __global__ void __launch_bounds__(xsp::NTHREADS, 1)
 k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
 {
@@ -142,8 +144,17 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
     constexpr int CPT = CB / NV;                      // channels per tile
     constexpr int SWP = 8 / CB;                       // row permutation: signal s of channel c in row s ^ SWP c
     constexpr uint32_t kIdesc = tc::idesc_f16(128, 64);
-    // FP16 range: 2-bit spectra reach 3.34 x 8192 = 2.7e4; 8-bit complex ones 180 x 4096 = 7.4e5, taken at 2^-5
-    constexpr float scale = CPX ? 0.03125f : 1.f;
+    // FP16's range.  2-bit spectra reach 3.34 x 8192 = 2.7e4; their weakest bins lie in FP32's own rounding of the FFT
+    // long before 2^-25, half of FP16's smallest step.  8-bit complex spectra reach 181.1 nchan and are taken at
+    // 256 / nchan, while a single unit sample in an FFT gives |X| = 1: up to 1024 channels its low part is still
+    // rounded no coarser than 2^-23 of it.  Beyond (WIDE) the low parts stand 2^LS higher, out of the subnormals, and
+    // go into D before the high parts, whose first product scales them back.  One unit sample per FFT, 64 FFTs, error
+    // of the worst baseline at 256 / 1024 / 4096 channels: 1.1e-6 each at a fixed 2^-5, now 2.4 / 3.0 / 2.8e-7
+    // (k_xplain 2.6 / 2.8 / 3.1e-7).  WIDE frees the tiles later: 24 antennas x 2 pol, 4096 channels, 800 FFTs
+    // 0.406 -> 0.456 ms.
+    constexpr bool CPX = IN != kReal, WIDE = IN == kComplexWide;
+    constexpr int LS = WIDE ? 10 : 0;
+    const float scale = CPX ? 256.f / (float)a.nchan : 1.f;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5;
@@ -271,18 +282,40 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                             const uint32_t d0 = tmem + db * 256;
                             uint32_t ds = dsm;
                             asm volatile("" : "+r"(ds));   // the descriptors are added up here, not kept
+                            auto hi = [&](int c, int h, int k) {   // K16 step k of part h: 32 bytes of the rows
+                                return udesc(ds + (uint32_t)((offsetof(Smem, hi) + c * HT) >> 4) + 2 * (KS * h + k));
+                            };
+                            auto lo = [&](int c, int h, int k) {
+                                return udesc(ds + (uint32_t)((offsetof(Smem, lo) + c * LT) >> 4) + 2 * (KS * h + k));
+                            };
+                            // a part's low products, then its high ones (WIDE: the low ones of all parts first)
 #pragma unroll
-                            for (int c = 0; c < NV; c++)
+                            for (int c = 0; c < NV; c++) {
 #pragma unroll
-                                for (int k = 0; k < 2 * KS; k++) {   // the low parts' steps, then the high ones'
-                                    // a K16 step: 32 bytes of the rows, + 2 in the descriptors' start field
-                                    const int at = 2 * (KS * h + k % KS);
-                                    const uint32_t dh = ds + (uint32_t)((offsetof(Smem, hi) + c * HT) >> 4) + at;
-                                    const uint32_t dl = ds + (uint32_t)((offsetof(Smem, lo) + c * LT) >> 4) + at;
-                                    if (h == 0 && k == 0) umma_ss_acc<false>(d0 + c * 64, udesc(dh), udesc(dl), kIdesc);
-                                    else umma_ss_acc<true>(d0 + c * 64, udesc(dh), udesc(k < KS ? dl : dh), kIdesc);
+                                for (int k = 0; k < KS; k++) {
+                                    if (h == 0 && k == 0) umma_ss_acc<false>(d0 + c * 64, hi(c, h, k), lo(c, h, k), kIdesc);
+                                    else umma_ss_acc<true>(d0 + c * 64, hi(c, h, k), lo(c, h, k), kIdesc);
                                 }
-                            umma_commit(&sm.empty16[h]);
+                                if constexpr (!WIDE)
+#pragma unroll
+                                    for (int k = 0; k < KS; k++)
+                                        umma_ss_acc<true>(d0 + c * 64, hi(c, h, k), hi(c, h, k), kIdesc);
+                            }
+                            if constexpr (!WIDE) {
+                                umma_commit(&sm.empty16[h]);
+                            } else if (h == NQ - 1) {
+#pragma unroll
+                                for (int g = 0; g < NQ; g++) {
+#pragma unroll
+                                    for (int c = 0; c < NV; c++)
+#pragma unroll
+                                        for (int k = 0; k < KS; k++) {
+                                            if (g == 0 && k == 0) umma_ss_scaled<LS>(d0 + c * 64, hi(c, g, k), hi(c, g, k), kIdesc);
+                                            else umma_ss_acc<true>(d0 + c * 64, hi(c, g, k), hi(c, g, k), kIdesc);
+                                        }
+                                    umma_commit(&sm.empty16[g]);
+                                }
+                            }
                             if (h == NQ - 1) umma_commit(&sm.d_full[db]);
                         }
                         __syncwarp();
@@ -323,7 +356,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                 const __half2 hh = __floats2half2_rn(v.x, v.y);
                 const float2 f = __half22float2(hh);
                 const float2 l = __fadd2_rn(v, make_float2(-f.x, -f.y));
-                const __half2 ll = __floats2half2_rn(l.x, l.y);
+                const __half2 ll = __floats2half2_rn(l.x * (float)(1 << LS), l.y * (float)(1 << LS));
                 hw[i] = h2(hh);
                 gw[i] = __byte_perm(hw[i], 0u, 0x1032) ^ 0x80000000u;   // (Im, -Re)
                 lw[i] = h2(__hadd2(ll, ll));
@@ -390,7 +423,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
         // columns of this warp's rows: all 64 signals, or the 32 of its own channel of the tile
         constexpr int NCOL = NS;
         const uint32_t lane0 = ((uint32_t)(q * 32) << 16) + (NS == 32 ? 32 * (q & 1) : 0);
-        constexpr float inv = 0.5f / (scale * scale) * (1.f + 0x1p-22f);   // what truncation took put back
+        const float inv = 0.5f * (1.f + 0x1p-22f) / (scale * scale);   // what truncation took put back
         const int nseg = (nk * BT + SEG - 1) / SEG;
         const int nd = nk / NQ;
         const int dseg = (nd + nseg - 1) / nseg;      // D per segment of an item
@@ -508,7 +541,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
     }
 }
 
-template <int NS, int NPOL, bool CPX>
+template <int NS, int NPOL, xsp::Input IN>
 static cudaError_t launch_xsplit_t(const XArgs& a, int* d_err, int nsm, cudaStream_t st)
 {
     using namespace xsp;
@@ -528,18 +561,21 @@ static cudaError_t launch_xsplit_t(const XArgs& a, int* d_err, int nsm, cudaStre
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
     const size_t sm = sizeof(Smem) + 1024;
     static unsigned configured = 0;
-    cudaError_t e = set_smem_once(k_xsplit<NS, NPOL, CPX>, sm, &configured);
+    cudaError_t e = set_smem_once(k_xsplit<NS, NPOL, IN>, sm, &configured);
     if (e != cudaSuccess) return e;
     const long long nitems = (long long)a.nsb * (a.nchan / CB);
     const int grid = nitems < nsm ? (int)nitems : nsm;
-    k_xsplit<NS, NPOL, CPX><<<grid, NTHREADS, sm, st>>>(map, a, d_err);
+    k_xsplit<NS, NPOL, IN><<<grid, NTHREADS, sm, st>>>(map, a, d_err);
     return cudaGetLastError();
 }
 
 template <int NS, int NPOL>
 static cudaError_t launch_xsplit_n(const XArgs& a, int cpx, int* d_err, int nsm, cudaStream_t st)
 {
-    return cpx ? launch_xsplit_t<NS, NPOL, true>(a, d_err, nsm, st) : launch_xsplit_t<NS, NPOL, false>(a, d_err, nsm, st);
+    using namespace xsp;
+    return !cpx            ? launch_xsplit_t<NS, NPOL, kReal>(a, d_err, nsm, st)
+           : a.nchan <= 1024 ? launch_xsplit_t<NS, NPOL, kComplex>(a, d_err, nsm, st)
+                             : launch_xsplit_t<NS, NPOL, kComplexWide>(a, d_err, nsm, st);
 }
 
 // A geometry-only rule (a batch's jobs take the same path as alone).  The kernel's time is that of an item,
