@@ -575,10 +575,10 @@ FArgs ctx_fargs(fxc_ctx* x, const uint8_t* d_data, size_t pitch, int ld)
     return a;
 }
 
-cudaError_t ctx_fstage(const fxc_ctx* x, const FArgs& fa, cudaStream_t st, int* nlaunch)
+cudaError_t ctx_fstage(const fxc_ctx* x, int mode, const FArgs& fa, cudaStream_t st, int* nlaunch)
 {
     if (nlaunch) *nlaunch = 1;
-    if (!x->d_turn) return launch_fstage(x->cfg.nchan, x->spec_mode, fa, st);
+    if (!x->d_turn) return launch_fstage(x->cfg.nchan, mode, fa, st);
     const int span = fa.tspan ? fa.tspan : fa.T;
     for (int s0 = 0; s0 < span; s0 += x->turn_T) {
         FArgs h = fa;
@@ -635,6 +635,8 @@ static int ctx_correlate(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const 
     }
     const bool tc = x->cfg.xmode != FXC_X_PLAIN_FP32;
     const bool fp8 = x->cfg.xmode == FXC_X_TC_FP8;
+    const bool xsplit = x->xsplit && nfft >= kXsplitMinFfts;
+    const int mode = x->xsplit && !xsplit ? (int)kSpecF32 : x->spec_mode;
     FArgs fa = ctx_fargs(x, d_data, pitch, ld);
     fa.amax = x->d_amax;
     XArgs xa{};
@@ -671,7 +673,7 @@ static int ctx_correlate(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const 
             StageScope sc(x, 1, 0);
             int n = 0;
             if (fp8) FXC_CK(cudaMemsetAsync(x->d_amax, 0, sizeof(unsigned) * xa.nsb * xa.nchan * xa.nsig, x->stream));
-            FXC_CK(ctx_fstage(x, fa, x->stream, &n));
+            FXC_CK(ctx_fstage(x, mode, fa, x->stream, &n));
             x->stage_launches[1] += n;
         }
         {
@@ -685,7 +687,7 @@ static int ctx_correlate(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const 
                 x8.inv_scale = x->d_inv;
                 FXC_CK(launch_xtc8(x8, x->d_err, x->nsm, x->stream));
             } else {
-                FXC_CK(x->xsplit ? launch_xsplit(xa, x->cfg.npol, x->cfg.iscomplex, x->d_err, x->nsm, x->stream)
+                FXC_CK(xsplit ? launch_xsplit(xa, x->cfg.npol, x->cfg.iscomplex, x->d_err, x->nsm, x->stream)
                        : !tc ? launch_xplain(xa, x->stream)
                            : x->spec_mode == kSpecH16 ? launch_xtch(xa, x->d_err, x->nsm, x->stream)
                                      : launch_xtc(xa, x->d_err, x->nsm, x->stream));
@@ -998,7 +1000,7 @@ int fxc_autotune(fxc_ctx* x, int reps)
     };
     // The F stage has no shape to choose (its slots draw FFT pairs from a counter; the FFT block only sets
     // a batch's task size): one run leaves the spectra the X stage's variants are timed on.
-    cudaError_t err = ctx_fstage(x, fa, x->stream);
+    cudaError_t err = ctx_fstage(x, x->spec_mode, fa, x->stream);
     float best = 1e30f;
     int best_alt = x->plan_alt;
     if (err == cudaSuccess && !tc && !x->xsplit) {

@@ -211,7 +211,7 @@ static int enqueue_launch(fxc_batch* b, const Launch& l)
         FB_CK(launch_fstage_batch(g.nchan, g.npol, g.mode, g.tb, b->d_fargs, b->d_tasks + l.task_off, l.ntask,
                                   b->ctx[0]->d_err + 2, b->stream));
     } else if (l.kind == kFJob) {
-        FB_CK(ctx_fstage(b->ctx[l.group], b->fa_host[(size_t)l.round * b->ctx.size() + l.group], b->stream));
+        FB_CK(ctx_fstage(b->ctx[l.group], b->ctx[l.group]->spec_mode, b->fa_host[(size_t)l.round * b->ctx.size() + l.group], b->stream));
     } else if (l.kind == kXGroup) {
         const XGroup& g = b->xg[l.group];
         FB_CK(launch_xplain_batch(g.nsig8 * 8, g.alt, b->d_xargs, b->d_tasks + l.task_off, l.ntask, b->stream));

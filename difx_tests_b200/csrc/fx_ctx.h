@@ -48,7 +48,7 @@ struct fxc_ctx {
     size_t acc_bytes = 0;
     void* d_xpart = nullptr;      // plain form with few channel groups: X-stage segment partial sums
     int xseg_max = 1;             // segments it holds
-    bool xsplit = false;          // plain form: X stage by launch_xsplit
+    bool xsplit = false;          // plain form: X stage by launch_xsplit (calls of kXsplitMinFfts FFTs and more)
     int* d_counts = nullptr;
     int* d_err = nullptr;   // device-side wait expiry code of the tensor-core X stage
     int nsm = 148;
@@ -106,7 +106,8 @@ int ctx_run_delay_table(fxc_ctx* x, const double* delays, const double* offs, in
                         const double* d_meta = nullptr);
 // F-stage arguments of this context for device input rows d_data of `pitch` bytes
 fx::FArgs ctx_fargs(fxc_ctx* x, const uint8_t* d_data, size_t pitch, int ld);
-// F stage of fa into the layout the context's X stage reads, on stream st; *nlaunch: kernels launched
-cudaError_t ctx_fstage(const fxc_ctx* x, const fx::FArgs& fa, cudaStream_t st, int* nlaunch = nullptr);
+// F stage of fa into spectra of layout mode (x->spec_mode, which the context's X stage reads, or kSpecF32 in its
+// place), on stream st; *nlaunch: kernels launched
+cudaError_t ctx_fstage(const fxc_ctx* x, int mode, const fx::FArgs& fa, cudaStream_t st, int* nlaunch = nullptr);
 // the plain X stage's time segments for xa (its nsig and alt set): tseg, tlen, part
 void ctx_xsegments(const fxc_ctx* x, fx::XArgs& xa);

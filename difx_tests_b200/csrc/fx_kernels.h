@@ -38,7 +38,9 @@ void xplain_segments(int nsig, int nchan, int nsb, int T, int nsm, int* tseg, in
 void xplain_segment_model(long long ctas, long long slots, int T, int* tseg, int* tlen);
 int xplain_segments_used(const XArgs& a);
 cudaError_t launch_xplain(const XArgs& a, cudaStream_t st);
-// whether the plain form of this geometry takes launch_xsplit (else launch_xplain)
+// whether the plain form of this geometry takes launch_xsplit (else launch_xplain); calls of fewer than
+// kXsplitMinFfts FFTs take launch_xplain either way
+constexpr int kXsplitMinFfts = 32;
 bool xsplit_pays(int nsig, int nchan, int nsb, int numffts, int nsm);
 // the plain form's sums on the tensor cores, FP32 values as exact FP16 pairs (up to 64 signals); cpx: 8-bit
 // complex input (spectra beyond FP16's range); spectra in the layout kSpecP32

@@ -585,11 +585,14 @@ static cudaError_t launch_xsplit_n(const XArgs& a, int cpx, int* d_err, int nsm,
 //       4096 FFTs, 9 signals (128 items) 210 / 204; 32 (128) 441 / 267; 33 (128) 400 / 235; 64 (512) 5683 / 2143
 //       and below, not: 9 (64) 117 / 203; 32 (96) 325 / 267; 33 (64) 206 / 234; 1024 FFTs, 9 (64) 41 / 59
 //   up to 8 signals k_xplain has little to do: 4096 FFTs (512) 290 / 699
+//   fewer FFTs than one D holds: what the truncations take is less than what is put back (1 FFT: error of the sums
+//       2.0e-7, 0.3e-7 on the FP32 units; 16: 1.4, 0.9; 24: 1.0, 1.1; 32: 0.9, 1.2)
 //   short calls of one item per SM: 64 FFTs, 2 signals (16) 23 / 13; 8 (128) 33 / 14; 64 (64) 45 / 23;
 //       not with more items: 2 (512) 24 / 25
 bool xsplit_pays(int nsig, int nchan, int nsb, int numffts, int nsm)
 {
     if (nsig < 1 || nsig > 64 || nchan < 8 || nchan % 8 != 0) return false;
+    if (numffts < kXsplitMinFfts) return false;
     const long long nitems = (long long)nsb * (nchan / (nsig <= 32 ? 8 : 4));
     if (numffts <= 128 && nitems <= nsm) return true;
     return nsig > 8 && nitems * 7 >= (long long)nsm * 6;
