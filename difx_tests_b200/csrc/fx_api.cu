@@ -622,9 +622,10 @@ void ctx_xsegments(const fxc_ctx* x, XArgs& xa)
     xa.part = xa.tseg > 1 ? x->d_xpart : nullptr;
 }
 
-// One call's correlation of device rows: whole subintegrations (win_base null) or windows.
+// One call's correlation of device rows: whole subintegrations (win_base null) or windows.  call_nfft: FFTs of the user's
+// call, of which these are all or a window's.
 static int ctx_correlate(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const double* d_meta,
-                         const double* delays, const double* offs, int first, int nfft)
+                         const double* delays, const double* offs, int first, int nfft, int call_nfft)
 {
     int ld = 0;
     {
@@ -635,7 +636,7 @@ static int ctx_correlate(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const 
     }
     const bool tc = x->cfg.xmode != FXC_X_PLAIN_FP32;
     const bool fp8 = x->cfg.xmode == FXC_X_TC_FP8;
-    const bool xsplit = x->xsplit && nfft >= kXsplitMinFfts;
+    const bool xsplit = x->xsplit && call_nfft >= kXsplitMinFfts;
     const int mode = x->xsplit && !xsplit ? (int)kSpecF32 : x->spec_mode;
     FArgs fa = ctx_fargs(x, d_data, pitch, ld);
     fa.amax = x->d_amax;
@@ -704,7 +705,7 @@ int fxc_process_device(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const do
 {
     if (!x || !d_data || pitch < x->subint + 16 || pitch % 16 || ((uintptr_t)d_data & 15)) return FXC_ERR_INVALID;
     FXC_CK(cudaSetDevice(x->device));
-    return ctx_correlate(x, d_data, pitch, nullptr, delays, offs, first, nfft);
+    return ctx_correlate(x, d_data, pitch, nullptr, delays, offs, first, nfft, nfft);
 }
 
 int fxc_process_device_window(fxc_ctx* x, const uint8_t* d_data, size_t pitch, const long long* base_sample,
@@ -722,7 +723,7 @@ int fxc_process_device_window(fxc_ctx* x, const uint8_t* d_data, size_t pitch, c
     double* d_meta = x->d_win_meta + (size_t)fxc_ctx::NWIN * 2 * c.nant;
     const int st = upload_window_meta(x, base_sample, len.data(), d_meta, x->stream);
     if (st != FXC_OK) return st;
-    return ctx_correlate(x, d_data, pitch, d_meta, delays, offs, first, nfft);
+    return ctx_correlate(x, d_data, pitch, d_meta, delays, offs, first, nfft, nfft);
 }
 
 }  // extern "C"
@@ -856,7 +857,7 @@ int fxc_process_host_window(fxc_ctx* x, const uint8_t* const* data, const double
         if (st != FXC_OK) return st;
         FXC_CK(cudaEventRecord(x->win_ready[s], x->copy_stream));
         FXC_CK(cudaStreamWaitEvent(x->stream, x->win_ready[s], 0));
-        st = ctx_correlate(x, x->d_win[s], x->win_pitch, d_meta, delays, offs, k, n);
+        st = ctx_correlate(x, x->d_win[s], x->win_pitch, d_meta, delays, offs, k, n, nfft);
         if (st != FXC_OK) return st;
         FXC_CK(cudaEventRecord(x->win_free[s], x->stream));
         k += n;

@@ -32,3 +32,21 @@ def test_short_call(nant, npol, nchan, numffts, nfft):
     want = np.array([[g[i * npol + l, j * npol + m] for l in range(npol) for m in range(npol)] for i, j in bls])
     # FP32 sums of nfft products: a unit roundoff of the products and half of one for each addition, at random
     assert np.linalg.norm(vis[0] - want) < U * (1 + 0.5 * nfft ** 0.5) * np.linalg.norm(want)
+
+
+@pytest.mark.gpu
+def test_short_last_window():
+    """Host rows go through the device in windows: a short last one takes the path of the whole call, as a short last
+    chunk of device rows does."""
+    job = synth.random_job(nant=12, npol=1, nchan=1024, numffts=70, bw=32e6, seed=3)
+    cfg = fx.make_config(12, 1024, 70, job.bw, job.lo, npol=1, chunk_ffts=64)
+    with fx.Correlator(cfg) as c:
+        c.process(job.data, job.delays, job.fileoffsets)
+        host = c.visibilities()
+        c.reset()
+        c.upload(job.data)
+        ptr, pitch = c.device_input()
+        c.process_device(ptr, pitch, job.delays, job.fileoffsets)
+        device = c.visibilities()
+    np.testing.assert_array_equal(host[1], device[1])
+    np.testing.assert_array_equal(host[0], device[0])
