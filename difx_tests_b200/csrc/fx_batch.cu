@@ -8,12 +8,13 @@
 //   channel-contiguous spectra, one F launch and corner turn per other job
 //   one k_xplain_batch launch per X group  {8-signal blocks, tile variant} (plain form, <= 64 signals),
 //   then one k_xplain_reduce per job of the group cut into time segments (as its single-job path cuts it)
-//   one X launch per remaining job: the FP16 tensor-core X stage, the plain X stage on the tensor cores
-//   (fx_xsplit.cu) or that of more than 64 signals
+//   one k_xsplit_batch launch per group {8-signal blocks, npol} of the plain jobs on the tensor cores
+//   one X launch per remaining job: the FP16 tensor-core X stage, or the plain X stage of more than 64 signals
 // A grouped launch works through a task table (F: persistent CTAs striding over it; plain X:
 // one CTA per task), so small and large jobs share the
 // machine inside one launch.  The delay tables and baseline counts run first.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -39,10 +40,14 @@ struct XGroup {
     int nsig8, alt;   // signal blocks of 8 (jobs with the same count share tile plans)
     std::vector<int> jobs;
 };
-enum LaunchKind { kFGroup = 0, kXGroup = 1, kXJob = 2, kXReduce = 3, kFJob = 4 };
+struct SGroup {
+    int nsig8, npol;  // signal blocks of 8 (the stages of a launch are laid out for its largest job)
+    std::vector<int> jobs;
+};
+enum LaunchKind { kFGroup = 0, kXGroup = 1, kXJob = 2, kXReduce = 3, kFJob = 4, kSGroup = 5 };
 struct Launch {       // one launch of the recorded sequence
     int kind;         // LaunchKind
-    int group;        // F / X group, or the job of a kXJob / kXReduce / kFJob launch
+    int group;        // F / X / S group, or the job of a kXJob / kXReduce / kFJob launch
     size_t task_off;  // into d_tasks (int4)
     int ntask;
     int round;        // kXJob / kXReduce / kFJob: the round (spectra chunk) whose arguments it takes
@@ -74,7 +79,8 @@ struct fxc_batch {
     cudaStream_t own = nullptr, stream = nullptr;
     std::vector<FGroup> fg;
     std::vector<XGroup> xg;
-    std::vector<int> job_fg, job_xg;   // -1: the job's F / X stage is its own launch
+    std::vector<SGroup> sg;
+    std::vector<int> job_fg, job_xg, job_sg;   // -1: not in such a group (in none: the stage is the job's own launch)
     std::vector<FArgs> fa_host;        // [nrounds][J], for the launches of one job
     std::vector<XArgs> xa_host;
     int nrounds = 0;
@@ -83,6 +89,9 @@ struct fxc_batch {
     XArgs* d_xargs = nullptr;
     int4* d_tasks = nullptr;
     size_t task_cap = 0;
+    // per job: 128 bytes of xsplit_map_bytes, error word (launch_xsplit_batch)
+    void* d_maps = nullptr;
+    int** d_errs = nullptr;
     std::vector<Launch> launches;
     bool tables_valid = false;
     // graph
@@ -181,14 +190,42 @@ static int build_tables(fxc_batch* b)
             if (tasks.size() > off) b->launches.push_back({kXGroup, g, off, (int)(tasks.size() - off), r});
             for (int j : segd) b->launches.push_back({kXReduce, j, 0, 0, r});
         }
+        for (int g = 0; g < (int)b->sg.size(); g++) {
+            // longest items first: a launch ends with short ones
+            std::vector<int> jobs;
+            for (int j : b->sg[g].jobs)
+                if (r < nchunks(b->ctx[j])) jobs.push_back(j);
+            std::stable_sort(jobs.begin(), jobs.end(),
+                             [&](int i, int j) { return chunk_span(b->ctx[i], r) > chunk_span(b->ctx[j], r); });
+            if (jobs.size() == 1) {
+                b->launches.push_back({kXJob, jobs[0], 0, 0, r});
+                continue;
+            }
+            const size_t off = tasks.size();
+            for (int j : jobs) {
+                const XArgs& xj = xa[(size_t)r * J + j];
+                for (int n = 0; n < xsplit_items(xj); n++) tasks.push_back(xsplit_item(xj, r * J + j, j, n));
+            }
+            if (tasks.size() > off) b->launches.push_back({kSGroup, g, off, (int)(tasks.size() - off), r});
+        }
         for (int j = 0; j < J; j++)
-            if (b->job_xg[j] < 0 && r < nchunks(b->ctx[j])) b->launches.push_back({kXJob, j, 0, 0, r});
+            if (b->job_xg[j] < 0 && b->job_sg[j] < 0 && r < nchunks(b->ctx[j])) b->launches.push_back({kXJob, j, 0, 0, r});
+    }
+    std::vector<std::array<char, 128>> maps(J);
+    std::vector<int*> errs;
+    for (int j = 0; j < J; j++) {
+        if (b->job_sg[j] >= 0) FB_CK(xsplit_map_bytes(xa[j], b->ctx[j]->cfg.npol, maps[j].data()));
+        errs.push_back(b->ctx[j]->d_err);
     }
     FB_CK(cudaSetDevice(b->device));
     cudaFree(b->d_fargs);
     cudaFree(b->d_xargs);
     b->d_fargs = nullptr;
     b->d_xargs = nullptr;
+    if (!b->d_maps) FB_CK(cudaMalloc(&b->d_maps, sizeof(maps[0]) * J));
+    if (!b->d_errs) FB_CK(cudaMalloc(&b->d_errs, sizeof(int*) * J));
+    FB_CK(cudaMemcpy(b->d_maps, maps.data(), sizeof(maps[0]) * J, cudaMemcpyHostToDevice));
+    FB_CK(cudaMemcpy(b->d_errs, errs.data(), sizeof(int*) * J, cudaMemcpyHostToDevice));
     if (tasks.size() > b->task_cap) {
         cudaFree(b->d_tasks);
         b->d_tasks = nullptr;
@@ -215,6 +252,10 @@ static int enqueue_launch(fxc_batch* b, const Launch& l)
     } else if (l.kind == kXGroup) {
         const XGroup& g = b->xg[l.group];
         FB_CK(launch_xplain_batch(g.nsig8 * 8, g.alt, b->d_xargs, b->d_tasks + l.task_off, l.ntask, b->stream));
+    } else if (l.kind == kSGroup) {
+        const SGroup& g = b->sg[l.group];
+        FB_CK(launch_xsplit_batch(std::min(64, 8 * g.nsig8), g.npol, b->d_xargs, b->d_maps, b->d_tasks + l.task_off, l.ntask,
+                                  b->ctx[0]->d_err + 2, b->d_errs, (int)b->ctx.size(), b->ctx[0]->nsm, b->stream));
     } else if (l.kind == kXReduce) {
         FB_CK(launch_xplain_reduce(b->xa_host[(size_t)l.round * b->ctx.size() + l.group], b->stream));
     } else {
@@ -288,12 +329,22 @@ int fxc_batch_create(const fxc_config* cfgs, int njobs, fxc_batch** out)
             b->fg[g].jobs.push_back(j);
         }
         b->job_fg.push_back(g);   // -1 for K-major spectra: its own F launches
-        if (c->cfg.xmode != FXC_X_PLAIN_FP32 || c->nsig > 64 || c->xsplit) {
-            b->job_xg.push_back(-1);   // its own X launch
-            continue;
-        }
         const int n8 = (c->nsig + 7) / 8;
         int h = -1;
+        if (c->xsplit) {
+            for (int k = 0; k < (int)b->sg.size(); k++)
+                if (b->sg[k].nsig8 == n8 && b->sg[k].npol == c->cfg.npol) h = k;
+            if (h < 0) {
+                b->sg.push_back({n8, c->cfg.npol, {}});
+                h = (int)b->sg.size() - 1;
+            }
+            b->sg[h].jobs.push_back(j);
+        }
+        b->job_sg.push_back(h);
+        if (c->cfg.xmode != FXC_X_PLAIN_FP32 || c->nsig > 64 || c->xsplit) {
+            b->job_xg.push_back(-1);
+            continue;
+        }
         for (int k = 0; k < (int)b->xg.size(); k++)
             if (b->xg[k].nsig8 == n8) h = k;
         if (h < 0) {
@@ -317,6 +368,8 @@ void fxc_batch_destroy(fxc_batch* b)
     cudaFree(b->d_fargs);
     cudaFree(b->d_xargs);
     cudaFree(b->d_tasks);
+    cudaFree(b->d_maps);
+    cudaFree(b->d_errs);
     if (b->own) cudaStreamDestroy(b->own);
     for (auto* c : b->ctx) fxc_destroy(c);
     delete b;

@@ -45,6 +45,15 @@ bool xsplit_pays(int nsig, int nchan, int nsb, int numffts, int nsm);
 // the plain form's sums on the tensor cores, FP32 values as exact FP16 pairs (up to 64 signals); cpx: 8-bit
 // complex input (spectra beyond FP16's range); spectra in the layout kSpecP32
 cudaError_t launch_xsplit(const XArgs& a, int npol, int cpx, int* d_err, int nsm, cudaStream_t st);
+// the same for the jobs of a batch (2-bit samples) in one launch.  Work item n of xsplit_items(a) of job `job`, whose
+// arguments are d_jobs[args]; 128 bytes per job of what the kernel reads its spectra by (at d_maps + 128 job, which is
+// 64-byte aligned); nsig_max: signals of the largest job, all of them up to 32 or all above; d_errs: every job's
+// error word
+int xsplit_items(const XArgs& a);
+int4 xsplit_item(const XArgs& a, int args, int job, int n);
+cudaError_t xsplit_map_bytes(const XArgs& a, int npol, void* map128);
+cudaError_t launch_xsplit_batch(int nsig_max, int npol, const XArgs* d_jobs, const void* d_maps, const int4* d_items,
+                                int nitems, int* ctr, int* const* d_errs, int njobs, int nsm, cudaStream_t st);
 cudaError_t launch_xplain_batch(int nsig, int alt, const XArgs* d_jobs, const int4* d_tasks, int ntask,
                                 cudaStream_t st);
 int xplain_channel_group(int nsig, int alt);

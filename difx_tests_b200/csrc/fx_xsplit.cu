@@ -54,6 +54,8 @@
 
 #include <cuda_fp16.h>
 
+#include <cstring>
+
 #include "fx_common.cuh"
 #include "fx_kernels.h"
 #include "fx_tc.cuh"
@@ -84,6 +86,12 @@ constexpr int TMEM_COLS = 512;               // two D: 4 x 64 columns each
 
 enum Input { kReal, kComplex, kComplexWide };   // 2-bit real samples; 8-bit complex, up to 1024 channels and beyond
 
+// An item of a batch's launch: what it takes from its job, and where its sums go (first subband and channel added)
+struct Item {
+    float2* acc;
+    int nsig, nchan, nk;
+};
+
 struct Smem {
     alignas(1024) uint8_t hi[NV * HT];
     alignas(1024) uint8_t lo[NV * LT];
@@ -98,6 +106,7 @@ struct Smem {
     uint64_t item_full[NITEM];
     uint64_t drain;
     int item[NITEM];                         // the CTA's items in order (nitems and more: no further one)
+    Item job[NITEM];                         // batch
     uint32_t tmem_base;
     int abort;
     int drain_fail;
@@ -132,11 +141,23 @@ __device__ __forceinline__ uint32_t h2(__half2 h) { return *reinterpret_cast<con
 
 }  // namespace xsp
 
+// The jobs of a batch's launch: items {job's arguments, subband, first channel, job}.  The stages of all jobs are laid
+// out for nsig signals.
+struct XBatch {
+    const XArgs* jobs;
+    const CUtensorMap* maps;     // of every job's spectra
+    const int4* items;
+    int nitems, nsig;
+    int* ctr;
+    int* const* err;             // every job's error word
+    int njobs;
+};
+
 // err: 1 a stage-full wait expired (cast or MMA); 2 a stage-free wait expired (producer or cast); 3 accumulator
 //      wait expired; 4 epilogue wait expired; 5 drain expired
-template <int NS, int NPOL, xsp::Input IN>
-__global__ void __launch_bounds__(xsp::NTHREADS, 1)
-k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
+// One job (map, a, err) or, BATCH, those of b.
+template <int NS, int NPOL, xsp::Input IN, bool BATCH>
+__device__ __forceinline__ void xsplit_cta(const CUtensorMap* tmap, const XArgs& a, int* err, const XBatch& b)
 {
     using namespace tc;
     using namespace xsp;
@@ -154,6 +175,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
     // 0.406 -> 0.456 ms.
     constexpr bool CPX = IN != kReal, WIDE = IN == kComplexWide;
     constexpr int LS = WIDE ? 10 : 0;
+    static_assert(!(BATCH && CPX), "a batch's jobs have 2-bit samples");
     const float scale = CPX ? 256.f / (float)a.nchan : 1.f;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -161,13 +183,17 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &sm.abort;
 
-    const int nsig = a.nsig;
-    const int npair = nsig * (nsig + 1) / 2;
-    const int ncg = a.nchan / CB;                 // channel groups per subband
-    const int nitems = a.nsb * ncg;
-    const int nk = (a.ntk ? a.ntk : a.T) / BT;    // stages per item (a multiple of NQ)
-    const uint32_t stage_bytes = (uint32_t)nsig * BT * CB * 8;
-    const int nst = min(MAXST, (int)(RING_BYTES / stage_bytes));
+    const int ncg = BATCH ? 1 : a.nchan / CB;     // channel groups per subband
+    const int nitems = BATCH ? b.nitems : a.nsb * ncg;
+    int* ctr = BATCH ? b.ctr : a.ctr;
+    const uint32_t stage_stride = (uint32_t)(BATCH ? b.nsig : a.nsig) * BT * CB * 8;
+    const int nst = min(MAXST, (int)(RING_BYTES / stage_stride));
+    // signals, channels and stages per item (a multiple of NQ)
+    Item one{nullptr, a.nsig, a.nchan, (a.ntk ? a.ntk : a.T) / BT};
+    auto from_args = [&](const XArgs& x, int sb, int c0) {
+        return Item{reinterpret_cast<float2*>(x.acc) + (size_t)sb * (x.nsig * (x.nsig + 1) / 2) * x.nchan + c0, x.nsig, x.nchan,
+                    (x.ntk ? x.ntk : x.T) / BT};
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < nst; s++) {
@@ -199,8 +225,16 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                    ? *reinterpret_cast<volatile int*>(&sm.item[n % NITEM])
                    : nitems;
     };
+    auto job_of = [&](int n) { return BATCH ? sm.job[n % NITEM] : one; };   // after item_of(n) gave an item
+    auto record = [&](int code) {
+        if constexpr (BATCH) {
+            for (int j = 0; j < b.njobs; j++) atomicCAS(b.err[j], 0, code);
+        } else {
+            atomicCAS(err, 0, code);
+        }
+    };
     auto fail = [&](int code) {
-        if (!*abort_flag) atomicCAS(err, 0, code);
+        if (!*abort_flag) record(code);
         *abort_flag = 1;
     };
 
@@ -215,21 +249,40 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                 // the first item by the block's number, the others from the counter: some SMs get a quarter less
                 // of the memory's rate than others
                 int item = blockIdx.x;
+                [[maybe_unused]] const CUtensorMap* mapped = nullptr;
                 for (int n = 0;; n++) {
                     if (*abort_flag) item = nitems;
+                    Item job = one;
+                    int sb, c0;
+                    const CUtensorMap* map = tmap;
+                    if constexpr (BATCH) {
+                        if (item < nitems) {
+                            const int4 it = b.items[item];
+                            sb = it.y;
+                            c0 = it.z;
+                            job = from_args(b.jobs[it.x], sb, c0);
+                            map = b.maps + it.w;
+                            sm.job[n % NITEM] = job;
+                            if (map != mapped)   // the copy of the map in global memory, before its first use
+                                asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+                            mapped = map;
+                        }
+                    } else {
+                        sb = item / ncg;
+                        c0 = (item - sb * ncg) * CB;
+                    }
                     sm.item[n % NITEM] = item;
                     mbar_arrive(&sm.item_full[n % NITEM]);
                     if (item >= nitems) break;
-                    const int next = nitems > (int)gridDim.x ? (int)gridDim.x + atomicAdd(a.ctr, 1) : nitems;
-                    const int sb = item / ncg;
-                    const int c0 = (item - sb * ncg) * CB;
-                    for (int kb = 0; kb < nk; kb++) {
+                    const int next = nitems > (int)gridDim.x ? (int)gridDim.x + atomicAdd(ctr, 1) : nitems;
+                    const uint32_t stage_bytes = (uint32_t)job.nsig * BT * CB * 8;
+                    for (int kb = 0; kb < job.nk; kb++) {
                         if (!mbar_wait(&sm.empty[stage], phase ^ 1, abort_flag)) {
                             fail(2);
                             break;
                         }
                         mbar_expect_tx(&sm.full[stage], stage_bytes);
-                        tma_load_4d(&tmap, &sm.full[stage], sm.ring + (size_t)stage * stage_bytes, 2 * c0,
+                        tma_load_4d(map, &sm.full[stage], sm.ring + (size_t)stage * stage_stride, 2 * c0,
                                     kb * (NPOL == 2 ? BT : BT / 2), 0, sb);
                         issued++;
                         if (++stage == nst) {
@@ -241,9 +294,9 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                 }
                 if (nitems > (int)gridDim.x) {   // the last CTA to have drawn leaves the counter zero
                     __threadfence();
-                    if (atomicAdd(a.ctr + 1, 1) == (int)gridDim.x - 1) {
-                        a.ctr[0] = 0;
-                        a.ctr[1] = 0;
+                    if (atomicAdd(ctr + 1, 1) == (int)gridDim.x - 1) {
+                        ctr[0] = 0;
+                        ctr[1] = 0;
                     }
                 }
                 // drain: the last nst fills are the only ones that may still be in flight
@@ -251,7 +304,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                     const long long idx = issued - 1 - s;
                     if (idx < 0) break;
                     if (!mbar_drain(&sm.full[(int)(idx % nst)], (uint32_t)((idx / nst) & 1))) {
-                        atomicCAS(err, 0, 5);
+                        record(5);
                         sm.drain_fail = 1;
                         break;
                     }
@@ -266,6 +319,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
             bool ok = true;
             for (int n = 0; ok; n++) {
                 if (item_of(n) >= nitems) break;
+                const int nk = job_of(n).nk;
                 for (int kb = 0; kb < nk && ok; kb += NQ) {
                     if (!mbar_wait_warp(&sm.d_empty[db], dph ^ 1, abort_flag)) {
                         if (lane == 0) fail(3);
@@ -329,7 +383,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
             if (elect_one()) {
                 umma_commit(&sm.drain);
                 if (!mbar_drain(&sm.drain, 0)) {
-                    atomicCAS(err, 0, 5);
+                    record(5);
                     sm.drain_fail = 1;
                 }
             }
@@ -343,7 +397,6 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
         const int tg = (lane / CB) & (NG - 1);
         constexpr int UPW = 32 / (NG * CB);               // units (a signal, or an antenna's two) of a warp at a time
         const int u0 = (warp - 4) * UPW + lane / (NG * CB);
-        const int nunit = nsig / NPOL;
         // two channels of a tile at NS = 32: rows H c0, H c1, H' c0, H' c1, so that its first 64 rows are B
         uint8_t* hi = sm.hi + (c / CPT) * HT + (c % CPT) * 32 * 128;
         uint8_t* lo = sm.lo + (c / CPT) * LT + (c % CPT) * 32 * 128;
@@ -373,6 +426,8 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
         bool stop = false;
         for (int n = 0; !stop; n++) {
             if (item_of(n) >= nitems) break;
+            const Item job = job_of(n);
+            const int nunit = job.nsig / NPOL, nk = job.nk;
             for (int kb = 0; kb < nk; kb++) {
                 const int h = kb & (NQ - 1);
                 if (!mbar_wait_warp(&sm.full[st], ph, abort_flag)) {
@@ -385,7 +440,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                     stop = true;
                     break;
                 }
-                const float4* src = reinterpret_cast<const float4*>(sm.ring + (size_t)st * stage_bytes) + tg * CB + c;
+                const float4* src = reinterpret_cast<const float4*>(sm.ring + (size_t)st * stage_stride) + tg * CB + c;
 #pragma unroll 2
                 for (int u = u0; u < nunit; u += NCW * UPW) {
                     if constexpr (NPOL == 2) {   // [ant][BT][chan] of both polarisations: FFTs tg + NG i
@@ -424,9 +479,6 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
         constexpr int NCOL = NS;
         const uint32_t lane0 = ((uint32_t)(q * 32) << 16) + (NS == 32 ? 32 * (q & 1) : 0);
         const float inv = 0.5f * (1.f + 0x1p-22f) / (scale * scale);   // what truncation took put back
-        const int nseg = (nk * BT + SEG - 1) / SEG;
-        const int nd = nk / NQ;
-        const int dseg = (nd + nseg - 1) / nseg;      // D per segment of an item
         int db = 0;
         uint32_t dph = 0;
         bool stop = false;
@@ -434,8 +486,11 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
             const int item = item_of(nit);
             // all of these warps leave together (a wait may have given up in one of them)
             if (bar_or(1, 32 * NEW, item >= nitems)) break;
-            const int sb = item / ncg;
-            const int c0 = (item - sb * ncg) * CB;
+            const Item job = BATCH ? job_of(nit) : from_args(a, item / ncg, item % ncg * CB);
+            const int nsig = job.nsig;
+            const int nseg = (job.nk * BT + SEG - 1) / SEG;
+            const int nd = job.nk / NQ;
+            const int dseg = (nd + nseg - 1) / nseg;      // D per segment of an item
             for (int d = 0; d < nd && !stop;) {
                 float2 sum[2][NCOL / 2];
 #pragma unroll
@@ -484,7 +539,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                         stop = bar_or(1, 32 * NEW, stop);
                         if (!stop) {
                             const int w = 4 * e + q;   // 0 .. 7
-                            float2* acc = reinterpret_cast<float2*>(a.acc) + (size_t)sb * npair * a.nchan + c0;
+                            float2* acc = job.acc;
                             if constexpr (NS == 32) {
                                 // channels 4 t + g, g = 0 .. 3: tile 2 t + (g >> 1)'s half g & 1; a thread takes channels
                                 // 4 t + 2 x and the next
@@ -503,7 +558,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                                         }
                                         const int p = i * nsig - i * (i - 1) / 2 + (j - i);
                                         asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(
-                                                         acc + (size_t)p * a.nchan + 4 * t + 2 * x),
+                                                         acc + (size_t)p * job.nchan + 4 * t + 2 * x),
                                                      "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3])
                                                      : "memory");
                                     }
@@ -519,7 +574,7 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
                                             const float vm = inv * (ig[(i ^ k) * VROW + (j ^ k)] - ig[(j ^ k) * VROW + (i ^ k)]);
                                             const int p = i * nsig - i * (i - 1) / 2 + (j - i);
                                             asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(
-                                                             acc + (size_t)p * a.nchan + ch),
+                                                             acc + (size_t)p * job.nchan + ch),
                                                          "f"(vr), "f"(vm)
                                                          : "memory");
                                         }
@@ -542,26 +597,48 @@ k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
 }
 
 template <int NS, int NPOL, xsp::Input IN>
+__global__ void __launch_bounds__(xsp::NTHREADS, 1)
+k_xsplit(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
+{
+    xsplit_cta<NS, NPOL, IN, false>(&tmap, a, err, XBatch{});
+}
+
+template <int NS, int NPOL>
+__global__ void __launch_bounds__(xsp::NTHREADS, 1)
+k_xsplit_batch(XBatch b)
+{
+    xsplit_cta<NS, NPOL, xsp::kReal, true>(nullptr, XArgs{}, nullptr, b);
+}
+
+// Spectra [sb][ant][T][chan][2 polarisations] or [sb][sig][T / 2][chan][2 FFTs] of 8-byte complex values
+static cudaError_t xsplit_map(const XArgs& a, int npol, CUtensorMap* map)
+{
+    using namespace xsp;
+    auto enc = tc::tensor_map_encoder();
+    if (!enc) return cudaErrorNotSupported;
+    const cuuint32_t cb = a.nsig <= 32 ? 8 : 4;
+    const cuuint64_t nt = npol == 2 ? a.T : a.T / 2, nr = a.nsig / npol, row = (cuuint64_t)a.nchan * 16;
+    const cuuint64_t dims[4] = {(cuuint64_t)2 * a.nchan, nt, nr, (cuuint64_t)a.nsb};
+    const cuuint64_t strides[3] = {row, nt * row, nr * nt * row};
+    const cuuint32_t box[4] = {2 * cb, (cuuint32_t)(npol == 2 ? BT : BT / 2), (cuuint32_t)nr, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 4, const_cast<void*>(a.spec), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+template <int NS, int NPOL, xsp::Input IN>
 static cudaError_t launch_xsplit_t(const XArgs& a, int* d_err, int nsm, cudaStream_t st)
 {
     using namespace xsp;
     constexpr int CB = 256 / NS;
-    auto enc = tc::tensor_map_encoder();
-    if (!enc) return cudaErrorNotSupported;
-    // spectra [sb][ant][T][chan][2 polarisations] or [sb][sig][T / 2][chan][2 FFTs] of 8-byte complex values
     CUtensorMap map;
-    const cuuint64_t nt = NPOL == 2 ? a.T : a.T / 2, nr = a.nsig / NPOL, row = (cuuint64_t)a.nchan * 16;
-    const cuuint64_t dims[4] = {(cuuint64_t)2 * a.nchan, nt, nr, (cuuint64_t)a.nsb};
-    const cuuint64_t strides[3] = {row, nt * row, nr * nt * row};
-    const cuuint32_t box[4] = {2 * CB, NPOL == 2 ? BT : BT / 2, (cuuint32_t)nr, 1};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_INT64, 4, const_cast<void*>(a.spec), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+    cudaError_t e = xsplit_map(a, NPOL, &map);
+    if (e != cudaSuccess) return e;
     const size_t sm = sizeof(Smem) + 1024;
     static unsigned configured = 0;
-    cudaError_t e = set_smem_once(k_xsplit<NS, NPOL, IN>, sm, &configured);
+    e = set_smem_once(k_xsplit<NS, NPOL, IN>, sm, &configured);
     if (e != cudaSuccess) return e;
     const long long nitems = (long long)a.nsb * (a.nchan / CB);
     const int grid = nitems < nsm ? (int)nitems : nsm;
@@ -598,17 +675,66 @@ bool xsplit_pays(int nsig, int nchan, int nsb, int numffts, int nsm)
     return nsig > 8 && nitems * 7 >= (long long)nsm * 6;
 }
 
-cudaError_t launch_xsplit(const XArgs& a, int npol, int cpx, int* d_err, int nsm, cudaStream_t st)
+static bool xsplit_fits(const XArgs& a, int npol)
 {
     using namespace xsp;
     const int nslot = a.ntk ? a.ntk : a.T;
-    if (a.nsig < 1 || a.nsig > 64 || a.nsig % npol || a.nchan % 8 != 0 || a.nchan < 8 || a.T % BT != 0 || nslot < 1 ||
-        nslot % (NQ * BT) != 0 || nslot > a.T || a.nsb < 1 || !a.spec || !a.acc)
-        return cudaErrorInvalidValue;
+    return a.nsig >= 1 && a.nsig <= 64 && a.nsig % npol == 0 && a.nchan % 8 == 0 && a.nchan >= 8 && a.T % BT == 0 && nslot >= 1 &&
+           nslot % (NQ * BT) == 0 && nslot <= a.T && a.nsb >= 1 && a.spec && a.acc;
+}
+
+cudaError_t launch_xsplit(const XArgs& a, int npol, int cpx, int* d_err, int nsm, cudaStream_t st)
+{
+    using namespace xsp;
+    if (!xsplit_fits(a, npol)) return cudaErrorInvalidValue;
     static_assert(sizeof(Smem) + 1024 <= 227 * 1024, "one CTA's shared memory");
     if (npol == 2)
         return a.nsig <= 32 ? launch_xsplit_n<32, 2>(a, cpx, d_err, nsm, st) : launch_xsplit_n<64, 2>(a, cpx, d_err, nsm, st);
     return a.nsig <= 32 ? launch_xsplit_n<32, 1>(a, cpx, d_err, nsm, st) : launch_xsplit_n<64, 1>(a, cpx, d_err, nsm, st);
+}
+
+// ---- a batch's jobs in one launch: the items of many short jobs fill the SMs together and share one start.  Whole
+// batch, a launch per job / one launch per group (one k_xplain launch): 32 jobs of 4 antennas x 128 channels x 100
+// FFTs 479 / 176 us (206); 64 of 16 antennas x 512 channels x 128 FFTs 1424 / 786 (1132); 12 of 9 antennas x 256
+// channels x 5 subbands x 2000 FFTs, whose items fill a last round of SMs badly alone, 3828 / 2752 (3296).
+int xsplit_items(const XArgs& a) { return a.nsb * (a.nchan / (a.nsig <= 32 ? 8 : 4)); }
+
+int4 xsplit_item(const XArgs& a, int args, int job, int n)
+{
+    const int cb = a.nsig <= 32 ? 8 : 4, ncg = a.nchan / cb;
+    return make_int4(args, n / ncg, n % ncg * cb, job);
+}
+
+cudaError_t xsplit_map_bytes(const XArgs& a, int npol, void* map128)
+{
+    static_assert(sizeof(CUtensorMap) == 128, "stride of the maps in memory");
+    if (!xsplit_fits(a, npol)) return cudaErrorInvalidValue;
+    CUtensorMap map;
+    const cudaError_t e = xsplit_map(a, npol, &map);
+    if (e == cudaSuccess) std::memcpy(map128, &map, sizeof map);
+    return e;
+}
+
+template <int NS, int NPOL>
+static cudaError_t launch_xsplit_batch_t(const XBatch& b, int nsm, cudaStream_t st)
+{
+    using namespace xsp;
+    const size_t sm = sizeof(Smem) + 1024;
+    static unsigned configured = 0;
+    const cudaError_t e = set_smem_once(k_xsplit_batch<NS, NPOL>, sm, &configured);
+    if (e != cudaSuccess) return e;
+    k_xsplit_batch<NS, NPOL><<<b.nitems < nsm ? b.nitems : nsm, NTHREADS, sm, st>>>(b);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_xsplit_batch(int nsig_max, int npol, const XArgs* d_jobs, const void* d_maps, const int4* d_items,
+                                int nitems, int* ctr, int* const* d_errs, int njobs, int nsm, cudaStream_t st)
+{
+    if (nsig_max < 1 || nsig_max > 64 || nitems < 1 || (npol != 1 && npol != 2)) return cudaErrorInvalidValue;
+    const XBatch b{d_jobs, static_cast<const CUtensorMap*>(d_maps), d_items, nitems, nsig_max, ctr, d_errs, njobs};
+    if (npol == 2)
+        return nsig_max <= 32 ? launch_xsplit_batch_t<32, 2>(b, nsm, st) : launch_xsplit_batch_t<64, 2>(b, nsm, st);
+    return nsig_max <= 32 ? launch_xsplit_batch_t<32, 1>(b, nsm, st) : launch_xsplit_batch_t<64, 1>(b, nsm, st);
 }
 
 }  // namespace fx
