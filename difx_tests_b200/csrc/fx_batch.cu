@@ -4,8 +4,9 @@
 //
 // Each job owns an ordinary context (device input, delay table, spectra chunk,
 // accumulators).  Per round r (spectra chunk r of every job that has one):
-//   one k_fpair_batch launch per F group {FFT length, npol, spectra layout} of the jobs whose X stage reads
-//   channel-contiguous spectra, one F launch and corner turn per other job
+//   one k_fpair_batch launch per F group {FFT length, npol, spectra layout}, and one k_kmajor_batch launch for the jobs
+//   whose X stage reads K-major spectra (their F stage writes channel-contiguous ones); F launches and corner turns
+//   of its own for a job of that kind with large chunks
 //   one k_xplain_batch launch per X group  {8-signal blocks, tile variant} (plain form, <= 64 signals),
 //   then one k_xplain_reduce per job of the group cut into time segments (as its single-job path cuts it)
 //   one k_xsplit_batch launch per group {8-signal blocks, npol} of the plain jobs on the tensor cores
@@ -33,7 +34,7 @@ using namespace fx;
 namespace {
 
 struct FGroup {
-    int nchan, npol, mode, tb;   // mode: the jobs' spectra layout (fxc_ctx::spec_mode)
+    int nchan, npol, mode, tb;   // mode: the layout the F stage writes (kSpecH16 also before a shared turn)
     std::vector<int> jobs;
 };
 struct XGroup {
@@ -44,11 +45,11 @@ struct SGroup {
     int nsig8, npol;  // signal blocks of 8 (the stages of a launch are laid out for its largest job)
     std::vector<int> jobs;
 };
-enum LaunchKind { kFGroup = 0, kXGroup = 1, kXJob = 2, kXReduce = 3, kFJob = 4, kSGroup = 5 };
+enum LaunchKind { kFGroup = 0, kXGroup = 1, kXJob = 2, kXReduce = 3, kFJob = 4, kSGroup = 5, kTurn = 6 };
 struct Launch {       // one launch of the recorded sequence
     int kind;         // LaunchKind
-    int group;        // F / X / S group, or the job of a kXJob / kXReduce / kFJob launch
-    size_t task_off;  // into d_tasks (int4)
+    int group;        // F / X / S group, the job of a kXJob / kXReduce / kFJob launch, the blocks of a kTurn launch
+    size_t task_off;  // into d_tasks (int4); kTurn: d_kjobs
     int ntask;
     int round;        // kXJob / kXReduce / kFJob: the round (spectra chunk) whose arguments it takes
 };
@@ -89,6 +90,7 @@ struct fxc_batch {
     XArgs* d_xargs = nullptr;
     int4* d_tasks = nullptr;
     size_t task_cap = 0;
+    KJob* d_kjobs = nullptr;     // corner turns of every round
     // per job: 128 bytes of xsplit_map_bytes, error word (launch_xsplit_batch)
     void* d_maps = nullptr;
     int** d_errs = nullptr;
@@ -135,6 +137,10 @@ static int build_tables(fxc_batch* b)
             a.t_base = r * c->T;
             a.nfft = std::min(c->T, c->cfg.numffts - r * c->T);
             a.tspan = chunk_span(c, r);
+            if (c->d_turn && b->job_fg[j] >= 0) {   // grouped: to the corner turn's input
+                a.spec = c->d_turn;
+                a.T = c->turn_T;
+            }
             fa[(size_t)r * J + j] = a;
         }
         XArgs x{};
@@ -156,6 +162,7 @@ static int build_tables(fxc_batch* b)
     b->fa_host = fa;
     b->xa_host = xa;
     std::vector<int4> tasks;
+    std::vector<KJob> kjobs;
     b->launches.clear();
     for (int r = 0; r < b->nrounds; r++) {
         for (int g = 0; g < (int)b->fg.size(); g++) {
@@ -171,8 +178,20 @@ static int build_tables(fxc_batch* b)
             }
             if (tasks.size() > off) b->launches.push_back({kFGroup, g, off, (int)(tasks.size() - off), r});
         }
-        for (int j = 0; j < J; j++)
-            if (b->job_fg[j] < 0 && r < nchunks(b->ctx[j])) b->launches.push_back({kFJob, j, 0, 0, r});
+        const size_t koff = kjobs.size();
+        int kblocks = 0;
+        for (int j = 0; j < J; j++) {
+            const fxc_ctx* c = b->ctx[j];
+            if (r >= nchunks(c)) continue;
+            if (b->job_fg[j] < 0) {
+                b->launches.push_back({kFJob, j, 0, 0, r});
+            } else if (c->d_turn) {
+                kjobs.push_back({c->d_turn, c->d_spec, c->turn_T, c->T, chunk_span(c, r), c->cfg.nsubband, c->nsig, c->cfg.nchan,
+                                 c->rows, kblocks});
+                kblocks += kmajor_blocks(kjobs.back());
+            }
+        }
+        if (kblocks) b->launches.push_back({kTurn, kblocks, koff, (int)(kjobs.size() - koff), r});
         for (int g = 0; g < (int)b->xg.size(); g++) {
             const size_t off = tasks.size();
             const int cg = xplain_channel_group(b->xg[g].nsig8 * 8, b->xg[g].alt);
@@ -220,8 +239,10 @@ static int build_tables(fxc_batch* b)
     FB_CK(cudaSetDevice(b->device));
     cudaFree(b->d_fargs);
     cudaFree(b->d_xargs);
+    cudaFree(b->d_kjobs);
     b->d_fargs = nullptr;
     b->d_xargs = nullptr;
+    b->d_kjobs = nullptr;
     if (!b->d_maps) FB_CK(cudaMalloc(&b->d_maps, sizeof(maps[0]) * J));
     if (!b->d_errs) FB_CK(cudaMalloc(&b->d_errs, sizeof(int*) * J));
     FB_CK(cudaMemcpy(b->d_maps, maps.data(), sizeof(maps[0]) * J, cudaMemcpyHostToDevice));
@@ -234,6 +255,8 @@ static int build_tables(fxc_batch* b)
     }
     FB_CK(cudaMalloc(&b->d_fargs, std::max<size_t>(1, fa.size()) * sizeof(FArgs)));
     FB_CK(cudaMalloc(&b->d_xargs, std::max<size_t>(1, xa.size()) * sizeof(XArgs)));
+    FB_CK(cudaMalloc(&b->d_kjobs, std::max<size_t>(1, kjobs.size()) * sizeof(KJob)));
+    if (!kjobs.empty()) FB_CK(cudaMemcpy(b->d_kjobs, kjobs.data(), kjobs.size() * sizeof(KJob), cudaMemcpyHostToDevice));
     FB_CK(cudaMemcpy(b->d_fargs, fa.data(), fa.size() * sizeof(FArgs), cudaMemcpyHostToDevice));
     FB_CK(cudaMemcpy(b->d_xargs, xa.data(), xa.size() * sizeof(XArgs), cudaMemcpyHostToDevice));
     FB_CK(cudaMemcpy(b->d_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice));
@@ -249,6 +272,8 @@ static int enqueue_launch(fxc_batch* b, const Launch& l)
                                   b->ctx[0]->d_err + 2, b->stream));
     } else if (l.kind == kFJob) {
         FB_CK(ctx_fstage(b->ctx[l.group], b->ctx[l.group]->spec_mode, b->fa_host[(size_t)l.round * b->ctx.size() + l.group], b->stream));
+    } else if (l.kind == kTurn) {
+        FB_CK(launch_kmajor_batch(b->d_kjobs + l.task_off, l.ntask, l.group, b->stream));
     } else if (l.kind == kXGroup) {
         const XGroup& g = b->xg[l.group];
         FB_CK(launch_xplain_batch(g.nsig8 * 8, g.alt, b->d_xargs, b->d_tasks + l.task_off, l.ntask, b->stream));
@@ -315,7 +340,14 @@ int fxc_batch_create(const fxc_config* cfgs, int njobs, fxc_batch** out)
     const auto plans = plan_cache_load();
     for (int j = 0; j < njobs; j++) {
         const fxc_ctx* c = b->ctx[j];
-        const int mode = c->spec_mode;   // the layout the job's X stage reads
+        // Jobs with K-major spectra share F and turn launches where their chunk is small: 24 jobs of 72 antennas x 128
+        // channels x 64 FFTs 768 us with launches of their own, 652 with shared ones; x 256 channels x 256 FFTs (19 MB)
+        // 1712 / 1560.  A larger chunk is better turned while L2 holds it: 24 x 72 antennas x 1024 channels x 256 FFTs
+        // (75 MB) 4117 / 4212.  Chunks turned in parts have launches of their own.
+        const int slots = std::min(c->T, (c->cfg.numffts + 63) / 64 * 64);
+        const bool turned = c->d_turn && c->turn_T >= slots &&
+                            4LL * c->nsb_g * c->nsig * c->cfg.nchan * slots <= (32 << 20);
+        const int mode = turned ? (int)kSpecH16 : c->spec_mode;
         int g = -1;
         for (int k = 0; k < (int)b->fg.size(); k++)
             if (b->fg[k].nchan == c->cfg.nchan && b->fg[k].npol == c->cfg.npol && b->fg[k].mode == mode) g = k;
@@ -328,7 +360,7 @@ int fxc_batch_create(const fxc_config* cfgs, int njobs, fxc_batch** out)
             }
             b->fg[g].jobs.push_back(j);
         }
-        b->job_fg.push_back(g);   // -1 for K-major spectra: its own F launches
+        b->job_fg.push_back(g);
         const int n8 = (c->nsig + 7) / 8;
         int h = -1;
         if (c->xsplit) {
@@ -368,6 +400,7 @@ void fxc_batch_destroy(fxc_batch* b)
     cudaFree(b->d_fargs);
     cudaFree(b->d_xargs);
     cudaFree(b->d_tasks);
+    cudaFree(b->d_kjobs);
     cudaFree(b->d_maps);
     cudaFree(b->d_errs);
     if (b->own) cudaStreamDestroy(b->own);

@@ -31,6 +31,15 @@ cudaError_t launch_ftc32(int mode, const FArgs& a, cudaStream_t st);
 // FP16 spectra [sb][sig][src_T][chan] -> K-major [sb][chan][rows][dst_T] from slot t_off on (fx_kmajor.cu)
 cudaError_t launch_kmajor(const void* src, int src_T, int span, int nsb, int nsig, int nchan, int rows, void* dst,
                           int dst_T, int t_off, unsigned* amax, cudaStream_t st);
+// the same for many jobs in one launch, each [sb][sig][src_T][chan] -> [sb][chan][rows][dst_T], slots [0, span)
+// (multiples of 64); first: blocks of the jobs before it
+struct KJob {
+    const void* src;
+    void* dst;
+    int src_T, dst_T, span, nsb, nsig, nchan, rows, first;
+};
+int kmajor_blocks(const KJob& j);
+cudaError_t launch_kmajor_batch(const KJob* d_jobs, int njobs, int nblocks, cudaStream_t st);
 cudaError_t launch_fstage_batch(int nchan, int npol, int mode, int tb, const FArgs* d_jobs, const int4* d_tasks,
                                 int ntask, int* ctr, cudaStream_t st);
 cudaError_t launch_xplain_reduce(const XArgs& a, cudaStream_t st);

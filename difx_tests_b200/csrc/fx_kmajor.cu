@@ -17,15 +17,16 @@ namespace {
 constexpr int KC = 64, KT = 64, KTHREADS = 256;
 }
 
-__global__ void __launch_bounds__(KTHREADS)
-k_kmajor(const __half2* __restrict__ src, int src_T, int nsig, int nchan, int rows, __half* __restrict__ dst, int dst_T,
-         int t_off, unsigned* __restrict__ amax)
+// FFTs KT tx .., channels KC cx .. of spectrum row z = (subband, signal)
+__device__ __forceinline__ void kmajor_tile(const __half2* __restrict__ src, int src_T, int nsig, int nchan, int rows,
+                                            __half* __restrict__ dst, int dst_T, int t_off, unsigned* __restrict__ amax,
+                                            int tx, int cx, int z)
 {
     __shared__ __align__(16) uint32_t tile[KT * KC];
-    const int t0 = blockIdx.x * KT, c0 = blockIdx.y * KC;
-    const int sb = blockIdx.z / nsig, sig = blockIdx.z - sb * nsig;
+    const int t0 = tx * KT, c0 = cx * KC;
+    const int sb = z / nsig, sig = z - sb * nsig;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const __half2* in = src + ((size_t)blockIdx.z * src_T + t0) * nchan + c0;
+    const __half2* in = src + ((size_t)z * src_T + t0) * nchan + c0;
     uint2 v[8];
 #pragma unroll
     for (int k = 0; k < 8; k++)
@@ -63,6 +64,37 @@ k_kmajor(const __half2* __restrict__ src, int src_T, int nsig, int nchan, int ro
             if (ch == 0 && f > 0.f) atomicMax(amax + item * nsig + sig, __float_as_uint(f));
         }
     }
+}
+
+__global__ void __launch_bounds__(KTHREADS)
+k_kmajor(const __half2* __restrict__ src, int src_T, int nsig, int nchan, int rows, __half* __restrict__ dst, int dst_T,
+         int t_off, unsigned* __restrict__ amax)
+{
+    kmajor_tile(src, src_T, nsig, nchan, rows, dst, dst_T, t_off, amax, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// Blocks [first, next job's first) turn a job's slots.
+__global__ void __launch_bounds__(KTHREADS) k_kmajor_batch(const KJob* __restrict__ jobs, int njobs)
+{
+    int lo = 0, hi = njobs - 1;
+    while (lo < hi) {
+        const int m = (lo + hi + 1) / 2;
+        if (jobs[m].first <= (int)blockIdx.x) lo = m;
+        else hi = m - 1;
+    }
+    const KJob& j = jobs[lo];
+    const int n = (int)blockIdx.x - j.first, nt = j.span / KT, nc = j.nchan / KC;
+    kmajor_tile(static_cast<const __half2*>(j.src), j.src_T, j.nsig, j.nchan, j.rows, static_cast<__half*>(j.dst), j.dst_T, 0,
+                nullptr, n % nt, n / nt % nc, n / nt / nc);
+}
+
+int kmajor_blocks(const KJob& j) { return j.span / KT * (j.nchan / KC) * j.nsb * j.nsig; }
+
+cudaError_t launch_kmajor_batch(const KJob* d_jobs, int njobs, int nblocks, cudaStream_t st)
+{
+    if (njobs < 1 || nblocks < 1) return cudaErrorInvalidValue;
+    k_kmajor_batch<<<nblocks, KTHREADS, 0, st>>>(d_jobs, njobs);
+    return cudaGetLastError();
 }
 
 // Slots [0, span) of src [nsb][nsig][src_T][nchan] to slots t_off .. of dst [nsb][nchan][rows][dst_T].
