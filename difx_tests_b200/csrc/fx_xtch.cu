@@ -14,8 +14,9 @@
 //
 // Persistent, warp-specialised CTA per SM; work item = (subband, CB channels): 8 channels (one whole
 // 32-byte sector of each spectrum row, N = 64 accumulator columns each) up to 32 signals, 4 channels
-// (N = 128) up to 64, which fills the 512 TMEM columns and 64 KB of operand tiles either way; with 4
-// the other half of a sector is the next item's, which another SM reads at the same time (L2):
+// (N = 128) up to 64, which fills the 512 TMEM columns and 64 KB of operand tiles either way, or 4 channels
+// (N = 64) for up to 32 signals of few channels; with 4 the other half of a sector is the next item's,
+// which another SM reads at the same time (L2):
 //   warp 0     TMA producer: box {CB channels, 32 FFTs, nsig signals} (unswizzled: (Re, Im) of the CB
 //              channels of FFT t of signal s at 4 CB (32 s + t)) into a ring of stages (as many as
 //              128 KB holds, up to 8)
@@ -47,10 +48,10 @@ constexpr int BT = 32;                       // FFTs per stage (a K half of the 
 constexpr int MAXSIG = 64;
 constexpr int RING_BYTES = 128 * 1024;       // stages of 4 CB BT nsig bytes
 constexpr int MAXST = 8;
-constexpr int TILES_BYTES = 64 * 1024;       // CB tiles of 512 / CB rows x 64 FP16
+constexpr int TILES_BYTES = 64 * 1024;       // CB tiles of N rows x 64 FP16
 constexpr int NTW = 8;                       // turn warps
 constexpr int NTHREADS = 32 * (2 + NTW + 4);   // producer, MMA, turn, 4 epilogue warps
-constexpr int TMEM_COLS = 512;               // CB channels x 512 / CB FP32 columns
+constexpr int TMEM_COLS = 512;               // CB channels x N FP32 columns
 
 struct Smem {
     alignas(1024) uint8_t f16[TILES_BYTES];
@@ -81,7 +82,7 @@ __device__ __forceinline__ void tma_load_4d(const CUtensorMap* map, uint64_t* ba
 
 // err: 0 ok; 1 a stage-full wait expired (turn or MMA); 2 a stage-free wait expired (producer or
 //      turn); 3 accumulator wait expired; 4 epilogue wait expired; 5 drain expired
-template <int CB>
+template <int CB, int N>
 __global__ void __launch_bounds__(tcxh::NTHREADS, 1)
 k_xtch(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
 {
@@ -93,7 +94,8 @@ k_xtch(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &sm.abort;
 
-    constexpr int N = 512 / CB;                   // accumulator columns (and tile rows) of a channel
+    // N: accumulator columns (and tile rows) of a channel
+    static_assert(CB * N <= TMEM_COLS && CB * N * 128 <= TILES_BYTES, "tiles and accumulators");
     constexpr int TILE_BYTES = N * 128;
     constexpr uint32_t kIdesc = tc::idesc_f16(128, N);
     const int nsig = a.nsig;
@@ -373,7 +375,7 @@ k_xtch(const __grid_constant__ CUtensorMap tmap, XArgs a, int* err)
     }
 }
 
-template <int CB>
+template <int CB, int N>
 static cudaError_t launch_xtch_t(const XArgs& a, int* d_err, int nsm, cudaStream_t st)
 {
     using namespace tcxh;
@@ -394,11 +396,11 @@ static cudaError_t launch_xtch_t(const XArgs& a, int* d_err, int nsm, cudaStream
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
     const size_t sm = sizeof(Smem) + 1024;
     static unsigned configured = 0;
-    cudaError_t e = set_smem_once(k_xtch<CB>, sm, &configured);
+    cudaError_t e = set_smem_once(k_xtch<CB, N>, sm, &configured);
     if (e != cudaSuccess) return e;
     const long long nitems = (long long)a.nsb * (a.nchan / CB);
     const int grid = nitems < nsm ? (int)nitems : nsm;
-    k_xtch<CB><<<grid, NTHREADS, sm, st>>>(map, a, d_err);
+    k_xtch<CB, N><<<grid, NTHREADS, sm, st>>>(map, a, d_err);
     return cudaGetLastError();
 }
 
@@ -410,7 +412,13 @@ cudaError_t launch_xtch(const XArgs& a, int* d_err, int nsm, cudaStream_t st)
         nslot > a.T || a.nsb < 1 || !a.spec || !a.acc)
         return cudaErrorInvalidValue;
     static_assert(sizeof(Smem) + 1024 <= 227 * 1024, "one CTA's shared memory");
-    return a.nsig <= 32 ? launch_xtch_t<8>(a, d_err, nsm, st) : launch_xtch_t<4>(a, d_err, nsm, st);
+    if (a.nsig > 32) return launch_xtch_t<4, 128>(a, d_err, nsm, st);
+    // Up to 32 signals, items of 4 channels (still 64 accumulator columns each) where one round of them is enough: an
+    // item of 8 takes 1.5 to 1.7 times as long, which pays only where it saves rounds.  128 to 512 channels, 4096
+    // FFTs, 8 / 4 channels: 4 signals 123 / 72 us, 16 113 / 78, 32 131 / 87; two rounds of 4, 1024 channels, 4 signals
+    // 123 / 163 (with 128 columns).
+    if ((long long)a.nsb * (a.nchan / 4) <= nsm) return launch_xtch_t<4, 64>(a, d_err, nsm, st);
+    return launch_xtch_t<8, 64>(a, d_err, nsm, st);
 }
 
 }  // namespace fx
