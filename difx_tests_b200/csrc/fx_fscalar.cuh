@@ -469,11 +469,10 @@ k_fscalar(FArgs args)
     fstage_block<F, TB, NPOL, CPX>(args, blockIdx.z, blockIdx.y, blockIdx.x * TB, smem, tw1, tw2, phase);
 }
 
-template <int F, int NPOL, bool CPX>
-cudaError_t launch_scalar(const FArgs& a, cudaStream_t st)
+template <int F, int TB, int NPOL, bool CPX>
+cudaError_t launch_scalar_tb(const FArgs& a, cudaStream_t st)
 {
     using P = SPlan<F, CPX>;
-    constexpr int TB = 16;
     const size_t sm = (size_t)P::NSLOT * P::BUF * sizeof(float2) + (P::TWREG ? 0 : (size_t)P::TWP * sizeof(float2)) +
                       (size_t)2 * P::NSLOT * P::NROT * sizeof(float2) + (size_t)(P::FS + P::FST) * sizeof(float) +
                       (size_t)P::NSLOT * 16 + (size_t)P::NSLOT * fstage_inb<F, NPOL, CPX>();
@@ -484,6 +483,24 @@ cudaError_t launch_scalar(const FArgs& a, cudaStream_t st)
     dim3 grid(((a.tspan ? a.tspan : a.T) + TB - 1) / TB, a.nant, a.nsb);
     kern<<<grid, P::NTHREADS, sm, st>>>(a);
     return cudaGetLastError();
+}
+
+template <int F, int NPOL, bool CPX>
+cudaError_t launch_scalar(const FArgs& a, cudaStream_t st)
+{
+    // A slot takes the FFTs of its block one after the other: in a short call blocks of 4 use more of the SMs.  16 / 4
+    // FFTs a block, us: 8 antennas x 64 FFTs of 8192 points 82 / 33, of 2048 28 / 17; 1024 points take the set-up of a
+    // block badly, so only what fits at once: 4 antennas x 256 FFTs 24 / 20, 12 x 256 30 / 34; full SMs 31 / 38.
+    if constexpr (F >= 1024) {
+        int dev = 0, nsm = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        const long long blocks = (long long)((a.nfft + 15) / 16) * a.nant * a.nsb;   // with FFTs
+        const long long cap = (long long)nsm * SPlan<F, CPX>::MINB;
+        if (F == 1024 ? 4 * blocks < cap : 3 * blocks < 2 * cap) return launch_scalar_tb<F, 4, NPOL, CPX>(a, st);
+    }
+    return launch_scalar_tb<F, 16, NPOL, CPX>(a, st);
 }
 
 template <int F>
