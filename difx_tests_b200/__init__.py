@@ -304,8 +304,8 @@ class Correlator:
         return tb.value, alt.value
 
     def autotune(self, reps=3):
-        """Pick the fastest F-stage FFT block and plain X tile variant on the current input and
-        delay model (needs one earlier process call); clears the accumulators."""
+        """Pick the fastest plain X tile variant (FP32 units) on the current input and delay model
+        (needs one earlier process call); clears the accumulators."""
         _check(_lib().fxc_autotune(self._ctx, reps), "fxc_autotune")
 
     def enable_stage_timing(self, on=True):

@@ -175,6 +175,12 @@ void plan_cache_append(const std::vector<std::string>& lines)
     }
 }
 
+void plan_line_if_new(const std::map<std::string, int>& file, const std::string& key, int value,
+                      std::vector<std::string>* lines)
+{
+    if (!file.count(key)) lines->push_back(key + " " + std::to_string(value));
+}
+
 static std::string fplan_key(const fxc_config& c)
 {
     return std::string(c.xmode == FXC_X_PLAIN_FP32 ? "F" : "H") + (c.iscomplex ? "C " : " ") +
@@ -1000,11 +1006,12 @@ int fxc_autotune(fxc_ctx* x, int reps)
         return cudaEventElapsedTime(ms, e0, e1);
     };
     // The F stage has no shape to choose (its slots draw FFT pairs from a counter; the FFT block only sets
-    // a batch's task size): one run leaves the spectra the X stage's variants are timed on.
-    cudaError_t err = ctx_fstage(x, x->spec_mode, fa, x->stream);
+    // a batch's task size): one run leaves the spectra the plain X stage's variants are timed on.
+    const bool timed = !tc && !x->xsplit;
+    cudaError_t err = timed ? ctx_fstage(x, x->spec_mode, fa, x->stream) : cudaSuccess;
     float best = 1e30f;
     int best_alt = x->plan_alt;
-    if (err == cudaSuccess && !tc && !x->xsplit) {
+    if (err == cudaSuccess && timed) {
         XArgs xa{};
         xa.spec = x->d_spec;
         xa.acc = x->d_acc;
@@ -1032,7 +1039,10 @@ int fxc_autotune(fxc_ctx* x, int reps)
         return FXC_ERR_CUDA;
     }
     x->plan_alt = best_alt;
-    plan_cache_append({fplan_key(c) + " " + std::to_string(x->plan_tb), xplan_key(x->nsig) + " " + std::to_string(best_alt)});
+    std::vector<std::string> lines;
+    plan_line_if_new(plan_cache_load(), fplan_key(c), x->plan_tb, &lines);
+    if (timed) lines.push_back(xplan_key(x->nsig) + " " + std::to_string(best_alt));
+    plan_cache_append(lines);
     return fxc_reset(x);   // the timing launches accumulated into the visibilities
 }
 

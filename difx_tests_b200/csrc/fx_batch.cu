@@ -1,6 +1,6 @@
 // fx_batch.cu -- many independent correlation jobs in grouped launches,
-// replayed as one CUDA graph, with an autotuner for the F-stage FFT
-// block size and the plain X-stage tile variant (include/fxcorr.h, fxc_batch_*).
+// replayed as one CUDA graph, with an autotuner for the plain X-stage
+// tile variant (include/fxcorr.h, fxc_batch_*).
 //
 // Each job owns an ordinary context (device input, delay table, spectra chunk,
 // accumulators).  Per round r (spectra chunk r of every job that has one):
@@ -65,10 +65,10 @@ thread_local int g_batch_cuda = 0;
         }                                                                                 \
     } while (0)
 
-// plan-cache keys as the single-job contexts write them ("F" FP32 spectra, "H" FP16)
+// plan-cache keys as the single-job contexts write them ("F" the plain form, "H" the tensor-core forms)
 std::string fkey(int nchan, int npol, int mode)
 {
-    return std::string(mode != kSpecF32 ? "H " : "F ") + std::to_string(2 * nchan) + " " + std::to_string(npol);
+    return std::string(mode != kSpecF32 && mode != kSpecP32 ? "H " : "F ") + std::to_string(2 * nchan) + " " + std::to_string(npol);
 }
 std::string xkey(int nsig8) { return "X " + std::to_string(nsig8); }
 
@@ -381,7 +381,7 @@ int fxc_batch_create(const fxc_config* cfgs, int njobs, fxc_batch** out)
             if (b->xg[k].nsig8 == n8) h = k;
         if (h < 0) {
             const auto it = plans.find(xkey(n8));
-            b->xg.push_back({n8, it != plans.end() ? it->second : 0, {}});
+            b->xg.push_back({n8, it != plans.end() && it->second == 1 ? 1 : 0, {}});
             h = (int)b->xg.size() - 1;
         }
         b->xg[h].jobs.push_back(j);
@@ -539,11 +539,11 @@ int fxc_batch_autotune(fxc_batch* b, int reps)
     FB_CK(cudaEventCreate(&e0));
     FB_CK(cudaEventCreate(&e1));
     int st = FXC_OK;
-    // time the round-0 launch of one group under each candidate plan
-    auto time_group = [&](int kind, int g, float* ms) -> int {
+    // time the round-0 launch of one X group under each candidate plan
+    auto time_group = [&](int g, float* ms) -> int {
         if (!b->tables_valid && (st = build_tables(b)) != FXC_OK) return st;
         for (const Launch& l : b->launches) {
-            if (l.kind != kind || l.group != g) continue;
+            if (l.kind != kXGroup || l.group != g) continue;
             if ((st = enqueue_launch(b, l)) != FXC_OK) return st;   // warm / sets attributes
             FB_CK(cudaEventRecord(e0, b->stream));
             for (int i = 0; i < reps; i++)
@@ -563,7 +563,7 @@ int fxc_batch_autotune(fxc_batch* b, int reps)
             b->xg[g].alt = alt;
             b->tables_valid = false;
             float ms = 0.f;
-            if ((st = time_group(kXGroup, g, &ms)) != FXC_OK) break;
+            if ((st = time_group(g, &ms)) != FXC_OK) break;
             if (ms < best_ms) {
                 best_ms = ms;
                 best = alt;
@@ -579,7 +579,8 @@ int fxc_batch_autotune(fxc_batch* b, int reps)
     if (st != FXC_OK) return st;
     {
         std::vector<std::string> lines;
-        for (const auto& g : b->fg) lines.push_back(fkey(g.nchan, g.npol, g.mode) + " " + std::to_string(g.tb));
+        const auto file = plan_cache_load();
+        for (const auto& g : b->fg) plan_line_if_new(file, fkey(g.nchan, g.npol, g.mode), g.tb, &lines);
         for (const auto& g : b->xg) lines.push_back(xkey(g.nsig8) + " " + std::to_string(g.alt));
         plan_cache_append(lines);
     }

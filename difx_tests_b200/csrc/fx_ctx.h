@@ -91,9 +91,14 @@ struct fxc_ctx {
 
 // Plan cache (file named by FXC_PLAN_CACHE): lines "<key...> <value>", later lines win.
 // Keys: "F <fft> <npol>" FFTs per F-stage task of the plain form, "H <fft> <npol>" of the tensor-core
-// forms, "X <signal blocks of 8>" plain X tile variant.
+// forms, "X <signal blocks of 8>" plain X tile variant.  The autotuners time the X variants and write those they
+// timed; nothing depends on the size of the F-stage tasks but the table they stand in, so it is written only where the
+// file has no entry.
 std::map<std::string, int> plan_cache_load();
 void plan_cache_append(const std::vector<std::string>& lines);
+// appends "<key> <value>" to lines unless the file has an entry of that key
+void plan_line_if_new(const std::map<std::string, int>& file, const std::string& key, int value,
+                      std::vector<std::string>* lines);
 
 // fxc_create with control over subband grouping (false: every subband in each chunk, as the
 // multi-job batch's task tables assume)

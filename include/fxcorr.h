@@ -229,11 +229,12 @@ int fxc_correlate_noalloc(const fxc_config* cfg, const uint8_t* d_data, size_t p
  * one CUDA graph of the whole sequence.  FXC_ERR_UNSUPPORTED for the FP8 form,
  * input windows, 8-bit complex input and the tensor-core F stages.
  * No counterpart in the reference (one job per run).
- * fxc_batch_autotune times the FFT block size (8/16/32 FFTs per task) of every
- * F group and the tile variant of every X group (the jobs on the FP32 units) on the uploaded data, keeps
- * the fastest, and zeroes the accumulators; with the environment variable
- * FXC_PLAN_CACHE naming a file, chosen plans are appended to it and read back by
- * later fxc_batch_create calls. */
+ * fxc_batch_autotune times the tile variant of every X group (the jobs on the FP32
+ * units) on the uploaded data, keeps the fastest, and zeroes the accumulators; with the
+ * environment variable FXC_PLAN_CACHE naming a file, the variants timed are appended to it
+ * and read back by later fxc_batch_create calls.  The FFT block (8/16/32 FFTs per F-stage
+ * task) only sets the size of the task table: it is not timed, and written where the file
+ * has no entry. */
 typedef struct fxc_batch fxc_batch;
 int fxc_batch_create(const fxc_config* cfgs, int njobs, fxc_batch** out);
 void fxc_batch_destroy(fxc_batch* b);
@@ -245,7 +246,7 @@ int fxc_batch_process(fxc_batch* b);
 int fxc_batch_reset(fxc_batch* b);
 int fxc_batch_get_visibilities(fxc_batch* b, int job, float* vis, int* counts, int normalize);
 int fxc_batch_autotune(fxc_batch* b, int reps);
-/* plan of a job's groups: FFTs per F-stage CTA and X tile variant (0/1) */
+/* plan of a job's groups: FFTs per F-stage task and X tile variant (0/1) */
 int fxc_batch_get_plan(fxc_batch* b, int job, int* fft_block, int* x_variant);
 int fxc_batch_set_stream(fxc_batch* b, void* stream);
 int fxc_batch_synchronize(fxc_batch* b);
@@ -262,9 +263,10 @@ int fxc_batch_launch_count(fxc_batch* b);
  * FFTs from a counter, whatever the first number. */
 int fxc_set_plan(fxc_ctx* ctx, int fft_block, int x_variant);
 int fxc_get_plan(fxc_ctx* ctx, int* fft_block, int* x_variant);
-/* Times every plan on the context's current input and delay model (at least one earlier
- * fxc_process_* call) with `reps` launches each, keeps the fastest, appends it to the plan cache
- * (when FXC_PLAN_CACHE is set) and clears the accumulators as fxc_reset does. */
+/* Times the tile variants of the plain X stage on the context's current input and delay model (at least
+ * one earlier fxc_process_* call) with `reps` launches each, keeps the fastest, appends it to the plan
+ * cache (when FXC_PLAN_CACHE is set) and clears the accumulators as fxc_reset does.  Contexts whose X
+ * stage is on the tensor cores have no variant to time. */
 int fxc_autotune(fxc_ctx* ctx, int reps);
 
 /* Per-stage device timing (the counterpart of the reference's per-stage clock()
