@@ -359,19 +359,6 @@ int ctx_create(const fxc_config* cfg, fxc_ctx** out, bool group_subbands)
     if ((e = cudaMalloc(&x->d_vbits, sizeof(uint32_t) * (size_t)c.nant * (x->ld / 32))) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&x->d_spec, x->spec_bytes)) != cudaSuccess) return fail(e);
     if ((e = cudaMemset(x->d_spec, 0, x->spec_bytes)) != cudaSuccess) return fail(e);
-    if (x->spec_mode == kSpecF16 && c.fstage != FXC_F_TC16 && c.fstage != FXC_F_TC32) {
-        // the FFT F stage's FP16 output before its corner turn: up to an eighth of the budget (2 GiB), in
-        // equal parts of the chunk; less where that much is not free
-        const size_t slot = G * x->nsig * (size_t)c.nchan * sizeof(uint32_t);
-        size_t part = std::max<size_t>(64, std::min(T, budget / 8 / slot / 64 * 64));
-        for (;; part = std::max<size_t>(64, part / 2 / 64 * 64)) {
-            const size_t n = (T + part - 1) / part;
-            x->turn_T = (int)round_up((T + n - 1) / n, 64);
-            if ((e = cudaMalloc(&x->d_turn, slot * x->turn_T)) == cudaSuccess) break;
-            if (e != cudaErrorMemoryAllocation || part == 64) return fail(e);
-            (void)cudaGetLastError();
-        }
-    }
     if (fp8) {
         const size_t n8 = x->spec_bytes / 2, nsc = (size_t)x->nsb_g * c.nchan * x->nsig;
         if ((e = cudaMalloc(&x->d_spec8, n8)) != cudaSuccess) return fail(e);
@@ -395,6 +382,21 @@ int ctx_create(const fxc_config* cfg, fxc_ctx** out, bool group_subbands)
     if ((e = cudaMalloc(&x->d_err, 4 * sizeof(int))) != cudaSuccess) return fail(e);
     if ((e = cudaMemset(x->d_err, 0, 4 * sizeof(int))) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&x->d_vis, x->vis_bytes)) != cudaSuccess) return fail(e);
+    if (x->spec_mode == kSpecF16 && c.fstage != FXC_F_TC16 && c.fstage != FXC_F_TC32) {
+        // the FFT F stage's FP16 output before its corner turn, in equal parts of the chunk: up to an eighth of the
+        // budget (2 GiB), and a quarter of what all the buffers that do not shrink left free
+        size_t free = 0, total = 0;
+        if ((e = cudaMemGetInfo(&free, &total)) != cudaSuccess) return fail(e);
+        const size_t slot = G * x->nsig * (size_t)c.nchan * sizeof(uint32_t);
+        size_t part = std::max<size_t>(64, std::min(T, std::min(budget / 8, free / 4) / slot / 64 * 64));
+        for (;; part = std::max<size_t>(64, part / 2 / 64 * 64)) {
+            const size_t n = (T + part - 1) / part;
+            x->turn_T = (int)round_up((T + n - 1) / n, 64);
+            if ((e = cudaMalloc(&x->d_turn, slot * x->turn_T)) == cudaSuccess) break;
+            if (e != cudaErrorMemoryAllocation || part == 64) return fail(e);
+            (void)cudaGetLastError();
+        }
+    }
 
     // constant tables: per-subband LO, f32 channel angular frequencies (kernel.c:162-166)
     std::vector<double> sblo(c.nsubband);
