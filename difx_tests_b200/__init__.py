@@ -366,8 +366,8 @@ class Correlator:
 
 
 class Batch:
-    """Many independent correlation jobs (each its own FxcConfig, plain FP32 X
-    form) processed by grouped persistent launches, replayed as one CUDA graph
+    """Many independent correlation jobs (each its own FxcConfig, plain FP32 or FP16
+    tensor-core X form) processed by grouped launches, replayed as one CUDA graph
     after the first call (fxc_batch_* of include/fxcorr.h)."""
 
     def __init__(self, cfgs):

@@ -11,8 +11,8 @@
 //   then one k_xplain_reduce per job of the group cut into time segments (as its single-job path cuts it)
 //   one k_xsplit_batch launch per group {8-signal blocks, npol} of the plain jobs on the tensor cores
 //   one X launch per remaining job: the FP16 tensor-core X stage, or the plain X stage of more than 64 signals
-// A grouped launch works through a task table (F: persistent CTAs striding over it; plain X:
-// one CTA per task), so small and large jobs share the
+// A grouped launch works through a task table (F: the table's pairs of FFTs drawn from a counter; plain X
+// on the FP32 units: one CTA per task; on the tensor cores: items drawn from a counter), so small and large jobs share the
 // machine inside one launch.  The delay tables and baseline counts run first.
 #include <algorithm>
 #include <array>

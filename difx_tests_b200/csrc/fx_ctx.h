@@ -33,7 +33,8 @@ struct fxc_ctx {
     uint32_t* d_vbits = nullptr;
     void* d_spec = nullptr;
     size_t spec_bytes = 0;
-    // X-stage input layout: kSpecF32 [sb][sig][T][chan] (the plain form), kSpecH16, the same in FP16 (the FP16
+    // X-stage input layout: kSpecF32 [sb][sig][T][chan] (the plain form on the FP32 units), kSpecP32, the F stage's two
+    // lanes side by side (the plain form on the tensor cores), kSpecH16, the first in FP16 (the FP16
     // tensor-core form of up to 64 signals on the FFT F stage, whose X stage turns the spectra on the
     // way into the MMA operand) or kSpecF16 K-major [sb][chan][rows][T] (the other tensor-core forms)
     int spec_mode = 0;

@@ -51,8 +51,8 @@ cudaError_t launch_xplain(const XArgs& a, cudaStream_t st);
 // kXsplitMinFfts FFTs take launch_xplain either way
 constexpr int kXsplitMinFfts = 32;
 bool xsplit_pays(int nsig, int nchan, int nsb, int numffts, int nsm);
-// the plain form's sums on the tensor cores, FP32 values as exact FP16 pairs (up to 64 signals); cpx: 8-bit
-// complex input (spectra beyond FP16's range); spectra in the layout kSpecP32
+// the plain form's sums on the tensor cores, each FP32 value as an FP16 pair of 22 bits (up to 64 signals); cpx:
+// 8-bit complex input (spectra beyond FP16's range); spectra in the layout kSpecP32
 cudaError_t launch_xsplit(const XArgs& a, int npol, int cpx, int* d_err, int nsm, cudaStream_t st);
 // the same for the jobs of a batch (2-bit samples) in one launch.  Work item n of xsplit_items(a) of job `job`, whose
 // arguments are d_jobs[args]; 128 bytes per job of what the kernel reads its spectra by (at d_maps + 128 job, which is

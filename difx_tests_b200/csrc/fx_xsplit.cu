@@ -1,5 +1,5 @@
-// fx_xsplit.cu -- plain X stage on the tensor cores at FP32 grade: every FP32 spectrum value as an FP16 pair,
-// exact products, and sums taken out of the tensor core every 32 FFTs.
+// fx_xsplit.cu -- plain X stage on the tensor cores at FP32 grade: every FP32 spectrum value as an FP16 pair of 22
+// bits, three of the four products, and sums taken out of the tensor core every 32 FFTs.
 //
 // Per channel V[i][j] = sum_t X_i conj(X_j) (kernel.c:829-854, conjugation of kernel.c:557-568 folded in).  With
 // x = h + l (h = FP16 rounding of x, l of the remainder; 22 bits), rows H = (Re, Im) and H' = (Im, -Re) of the
@@ -12,7 +12,9 @@
 // off every visibility, over 64 FFTs 5e-7, over 32 (two additions of low parts, two of high ones, twice) 2.5e-7.
 // So D holds 32 FFTs only; then the epilogue warps add it, rounded to nearest, to running sums in their registers,
 // while the MMAs fill the other D, and the mean of what the truncations took, 2^-22, is put back on the way
-// out.  After 2048 FFTs at most the sums go to the accumulators: additions to a small sum round less than to a
+// out: the mean over Gaussian samples and whole D.  The last D of a call may hold fewer FFTs and lose less (its share
+// of the sums is too large by up to 1.5e-7), and sums of few bits lose nothing; calls of less than one D go to
+// k_xplain.  After 2048 FFTs at most the sums go to the accumulators: additions to a small sum round less than to a
 // large one.  Error of the whole correlation against 64 bits, k_xplain / here (without the 2^-22 / D of
 // 16 FFTs with 2^-23 put back, which is 5 % slower):
 //     4 antennas x 2 pol, 128 channels, 100 FFTs                               1.4 / 1.0e-7 (2.7 / 0.9e-7)
@@ -658,9 +660,16 @@ static cudaError_t launch_xsplit_n(const XArgs& a, int cpx, int* d_err, int nsm,
 // A geometry-only rule (a batch's jobs take the same path as alone).  The kernel's time is that of an item,
 // 10 us + 0.042 (2 signals) to 0.07 us (64) per FFT, times the items over the SMs; k_xplain's grows with the
 // multiply-adds but takes 23 us or more.  Measured k_xplain / here, us (items):
-//   9 to 64 signals, items for most SMs: here the faster one for every number of FFTs tried
-//       4096 FFTs, 9 signals (128 items) 210 / 204; 32 (128) 441 / 267; 33 (128) 400 / 235; 64 (512) 5683 / 2143
-//       and below, not: 9 (64) 117 / 203; 32 (96) 325 / 267; 33 (64) 206 / 234; 1024 FFTs, 9 (64) 41 / 59
+//   17 to 64 signals, items for most SMs: here, also with a last round of items that is nearly empty
+//       4096 FFTs, 17 signals (128) 389 / 213, (160) 490 / 414; 32 (128) 443 / 261, (160) 556 / 509, (320) 1083 / 763;
+//       33 (160) 506 / 439; 64 (160) 959 / 553, (512) 5683 / 2143; below, not: 32 (64) 226 / 256; 33 (64) 207 / 224
+//   9 to 16 signals: the faster one where every round of items is 6/7 full (an item is not cut)
+//       4096 FFTs, 9 signals (128) 210 / 198, (288) 445 / 387; 16 (128) 234 / 203; 512 FFTs, 12 (288) 72 / 61
+//     where it is not, the slower one by up to 1.45 (a batch's jobs share rounds), and still chosen: its sums are the
+//     more accurate (9 signals, 160 items, 4096 FFTs 1.1e-7, k_xplain 2.2e-7)
+//       4096 FFTs, 9 signals (160) 264 / 385, (224) 364 / 390, (320) 498 / 566, (448) 693 / 751; 16 (192) 338 / 394,
+//       (320) 558 / 579; 512 FFTs, 12 (160) 50 / 58, (192) 57 / 59
+//     with half of the SMs idle, not: 9 (64) 117 / 195; 1024 FFTs, 9 (64) 41 / 59
 //   up to 8 signals k_xplain has little to do: 4096 FFTs (512) 290 / 699
 //   fewer FFTs than one D holds: what the truncations take is less than what is put back (1 FFT: error of the sums
 //       2.0e-7, 0.3e-7 on the FP32 units; 16: 1.4, 0.9; 24: 1.0, 1.1; 32: 0.9, 1.2)

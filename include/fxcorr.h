@@ -43,9 +43,11 @@ extern "C" {
 #define FXC_ERR_TIMEOUT      -6   /* a bounded device-side wait expired; that call's result is invalid */
 
 /* X-stage arithmetic */
-#define FXC_X_PLAIN_FP32 0        /* FP32 cross-multiply-accumulate: on the FP32 units or, with up to 64 signals and
-                                     enough channels, on the tensor cores (each FP32 value as two FP16 ones, FP32
-                                     sums flushed every 16 FFTs: FP32-grade results, chosen by geometry) */
+#define FXC_X_PLAIN_FP32 0        /* FP32 cross-multiply-accumulate: on the FP32 units or, with up to 64 signals,
+                                     enough channels and calls of 32 FFTs or more, on the tensor cores (each FP32
+                                     value as two FP16 ones, 22 bits together, their accumulators added to FP32
+                                     sums every 32 FFTs: errors no larger than on the FP32 units; chosen by
+                                     geometry and call length) */
 #define FXC_X_TC_FP16    1        /* tcgen05 tensor cores, FP16 inputs, FP32 accumulation (on the FFT F
                                      stage with <= 64 signals the X stage turns the FP16 spectra itself;
                                      FXC_TC_SPECTRA=f16 in the environment at context creation has them
@@ -205,7 +207,8 @@ int fxc_host_free(void* p);
  * FXC_NOALLOC_SCRATCH_BYTES that each GPU loading this library holds until the
  * process exits; a problem whose delay table, accumulators and at least 64 FFT
  * slots of spectra do not fit returns FXC_ERR_INVALID.  Plain FP32 X stage only
- * (FXC_ERR_UNSUPPORTED otherwise).  Work is queued on `stream` (a cudaStream_t,
+ * (FXC_ERR_UNSUPPORTED otherwise), on the FP32 units: where fxc_process_device takes the
+ * tensor cores its results differ from these in the last bits.  Work is queued on `stream` (a cudaStream_t,
  * NULL = legacy default stream); the call returns before it completes, so a
  * device wait that runs out is reported in the outputs instead: every
  * visibility NaN and every count -6.  All calls share the array: calls that overlap on the GPU race, so order them (one
@@ -220,10 +223,12 @@ int fxc_correlate_noalloc(const fxc_config* cfg, const uint8_t* d_data, size_t p
  * subbands, subintegration length) and X form (plain FP32 or FP16 tensor cores).
  * fxc_batch_process runs every job's whole subintegration: one persistent
  * F-stage launch per group of jobs sharing FFT length, polarisation count and
- * spectra precision (CTAs stride over a task table of {job, subband, antenna
- * block}), one plain X-stage launch per group of jobs of at most 64 signals
- * sharing an X tile plan (one CTA per {job, subband, channel block} task), and
- * one X launch per other job (FP16
+ * spectra layout (its FFTs are drawn from a table of {job, subband, antenna, first
+ * FFT} tasks), one corner turn for the FP16 jobs of more than 64 signals (those with
+ * large chunks have F launches and turns of their own), one plain X-stage launch per
+ * group of jobs of at most 64 signals that share an X tile plan (on the FP32 units, one
+ * CTA per {job, subband, channel block} task) or their number of signals in blocks of 8
+ * and of polarisations (on the tensor cores), and one X launch per other job (FP16
  * tensor-core jobs, plain jobs of more than 64 signals), in rounds when a job
  * needs several spectra chunks.  The first call runs eagerly; later calls replay
  * one CUDA graph of the whole sequence.  FXC_ERR_UNSUPPORTED for the FP8 form,
