@@ -411,6 +411,22 @@ def spectra_f16(xmode, fstage, w):
                 and w["nchan"] % 4 == 0 and os.environ.get("FXC_TC_SPECTRA") != "f16")
 
 
+def f_turned(xmode, fstage, w):
+    """Whether the F stage is an FFT kernel and a corner turn (k_kmajor) of its FP16 spectra."""
+    return fstage in (0, 1) and spectra_f16(xmode, fstage, w)
+
+
+def f_kernel(xmode, fstage, w):
+    """What the F stage's launches are, for the roofline line."""
+    import difx_tests_b200 as fx
+    name = F_KERNELS[fstage]
+    if xmode == fx.FXC_X_TC_FP8 and fstage in (0, 1):
+        name = "k_fscalar (fused unpack/shift/fringe/FFT/frac-delay, one scalar FP32 FFT per slot on the CUDA cores)"
+    if f_turned(xmode, fstage, w):
+        name += " and k_kmajor (corner turn of its FP16 spectra), the two as one launch"
+    return name
+
+
 def form_dtype(form, w):
     """dtype label of the form as it runs on w (a tensor-core F form that fell back reads as tc)."""
     return DTYPES[form] if form_params(form, w) == FORMS[form] else DTYPES["tc"]
@@ -466,7 +482,8 @@ def time_form(torch, dist, fx, w, form, data, pitch, delays, offs, steps, warmup
     corr.enable_stage_timing(False)
     from difx_tests_b200 import sharding
     ms_max = sharding.max_over_ranks(ms, device=dev)   # device time: max over ranks
-    f_launches = max(1, int(launches[1]))
+    # an FFT kernel and its corner turn count as one launch of the F stage
+    f_launches = max(1, int(launches[1]) // (2 if f_turned(xmode, fstage, w) else 1))
     x_launches = max(1, int(launches[2]))
     ffts_per_launch = w["numffts"] * steps / f_launches
     samples_per_launch = nsig * w["nsb"] * ffts_per_launch * F
@@ -527,12 +544,13 @@ def run_gpu_arm(args):
     # ---- roofline of the dominant kernel of the headline form (the F stage)
     hbm, tc_peak, peak_kind = peaks()
     f16 = xmode != 0                 # the plain form's spectra are FP32
-    spec_bpc = 4 if f16 else 8       # bytes per complex spectrum value written
+    # bytes per complex spectrum value written; a corner turn reads and writes FP16 ones once more
+    spec_bpc = 12 if f_turned(xmode, fstage, w) else 4 if f16 else 8
     f_bytes = head["samples_per_launch"] * (0.25 + 0.5 * spec_bpc)
     f_gbs = f_bytes / (head["f_ms_launch"] / 1e3) / 1e9
     sm = head["stage_ms"]
     dram = FSTAGE_DRAM_BYTES_PER_SAMPLE.get((fstage, f16)) if w["nchan"] == 1024 else None
-    roof = {"kernel": F_KERNELS[fstage] + (", FP16 spectra out" if f16 else ", FP32 spectra out"),
+    roof = {"kernel": f_kernel(xmode, fstage, w) + (", FP16 spectra out" if f16 else ", FP32 spectra out"),
             "bound": "hbm", "achieved": f_gbs,
             "peak": hbm, "unit": "GB/s", "frac": f_gbs / hbm,
             "traffic": dram * head["samples_per_launch"] if dram else None,
@@ -541,6 +559,8 @@ def run_gpu_arm(args):
             "share": sm[1] / max(1e-9, sm.sum()),
             "note": ("latency-bound warp-specialised pipeline; HBM fraction shown for its algorithmic bytes"
                      if fstage in (2, 3) else
+                     "scalar FP32 FFT is bound by instruction issue; HBM fraction shown for its algorithmic bytes"
+                     if xmode == fx.FXC_X_TC_FP8 else
                      "FP32 FFT is bound by shared memory and the FP32 pipe; HBM fraction shown for its algorithmic bytes")}
 
     line = {
