@@ -359,8 +359,9 @@ def run_reference_arm(args):
 # DRAM bytes per input sample of the F-stage kernels (2048-point FFTs), dram__bytes_read.sum +
 # dram__bytes_write.sum from one ncu capture each on the 64-antenna x 1024-channel profiling case,
 # divided by the samples of that launch: key (fstage, F16 output)
-# (profiles/k_ftc_cfg2s_ncu.txt for k_ftc, profiles/k_ftc32_cfg2s_ncu.txt for k_ftc32; none of k_fpair).
-FSTAGE_DRAM_BYTES_PER_SAMPLE = {(2, True): 2.17, (3, True): 2.18}
+# (profiles/k_ftc_cfg2s_ncu.txt for k_ftc, profiles/k_ftc32_cfg2s_ncu.txt for k_ftc32, profiles/k_fpair_ncu.txt
+# for k_fpair, FP32 spectra only).
+FSTAGE_DRAM_BYTES_PER_SAMPLE = {(1, False): 4.16, (2, True): 2.17, (3, True): 2.18}
 
 
 # form -> (fxc_config.xmode, fxc_config.fstage)

@@ -6,8 +6,8 @@
 //   unnormalised FFT (499-510), fractional-sample correction (512-555), store of channels [0, C).
 //   The conjugation (557-568) is folded into the X stage.
 //
-// What bounds it: shared memory (exchanges, twiddles, sample table: 400 to 455 wavefronts per 1024
-// samples, 75 % of the data pipe), then the FP32 pipe (50 %); HBM runs at a quarter of its rate.  A
+// What bounds it: shared memory (exchanges, twiddles, sample table: 401 wavefronts per 1024 samples at 4096
+// points, 73 % of the data pipe), then the FP32 pipe (53 %); HBM runs at a quarter of its rate.  A
 // scalar FFT is bound by instruction issue instead (75 instructions per sample).  So a slot of NT = F / 16 threads takes a PAIR of FFTs -- both polarisations
 // of one FFT, or two consecutive FFTs of a single-polarisation antenna -- and holds 16 points of
 // each as (lane A, lane B) register pairs: every butterfly is a packed f32x2 instruction on two
@@ -49,7 +49,7 @@
 //
 // Real samples at 1024 and 2048 points (PPlan::R32) take a plan with one exchange instead of two: 32 points a thread
 // (32 x 32; 64 x 32 with two threads to a set of 64 samples, each of which decodes all of them and forms its half of
-// stage 0's outputs), 290 wavefronts per 1024 samples instead of 400 to 455, one barrier fewer, coalesced runs of 32
+// stage 0's outputs), 314 wavefronts per 1024 samples (2048 points), one barrier fewer, coalesced runs of 32
 // channels.  It costs 184 registers, so 8 warps per SM: too few to hide a pair's preparation, which a helper warp
 // per slot does instead -- descriptors in registers, samples straight from global memory, factor
 // tables three FP64 chains abreast -- and meets the slot's threads at two barriers per pair:

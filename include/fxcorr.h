@@ -83,7 +83,7 @@ typedef struct fxc_config {
  * (kernel.c:499-510, IPP ippsFFTFwd_CToC_32fc); every choice but FXC_F_TC16 keeps FP32
  * accuracy.  The X forms read the F stage's output as FP32 (plain) or cast to FP16 / e4m3
  * (tensor-core forms).
- *   FXC_F_AUTO   FXC_F_FFT32.
+ *   FXC_F_AUTO   FXC_F_FFT32, the fastest at FP32 accuracy.
  *   FXC_F_FFT32  FP32 radix-16 Stockham FFT on the CUDA cores; every geometry and form.
  *   FXC_F_TC16   FP16 DFT on the tensor cores: the 2048-point FFT as two tcgen05 GEMMs with
  *                FP16 DFT matrices and an FP16 intermediate (three FP16 roundings inside the
