@@ -12,9 +12,9 @@ pytestmark = pytest.mark.gpu
 
 def test_little_memory(monkeypatch):
     monkeypatch.setenv("FXC_SPECTRA_BUDGET_MB", "4096")
-    nant, nchan, numffts = 128, 4096, 300
-    # 320 slots in two parts of 160 with room enough
-    turn = 160 * nant * nchan * 4
+    nant, nchan, numffts = 128, 4096, 900
+    # with room enough the 960 slots are turned 256 at a time; 64 at a time need a quarter of that
+    turn = 256 * nant * nchan * 4
     job = synth.random_job(nant=nant, npol=1, nchan=nchan, numffts=numffts, bw=32e6, seed=1)
     cfg = fx.make_config(nant, nchan, numffts, job.bw, job.lo, npol=1, xmode=fx.FXC_X_TC_FP16)
 
